@@ -796,7 +796,6 @@ static b2f_status add_bluestein_large(Builder& b, int axis, uint64_t N, uint64_t
   const uint64_t M = bluestein_length(b, N);
   const uint64_t nlines = s * O;
   b.need(BUF_WS2, nlines * M * b.cb());
-  b.need(dst, N * s * O * b.cb());
   Pass pre;
   pre.kind = Pass::BLUE_ELEM;
   pre.axis = axis;
@@ -846,7 +845,6 @@ static b2f_status add_rader_large(Builder& b, int axis, uint64_t p, uint64_t s, 
   const uint64_t M = p - 1;
   const uint64_t nlines = s * O;
   b.need(BUF_WS2, nlines * M * b.cb());
-  b.need(dst, p * s * O * b.cb());
   const uint64_t g = primitive_root(p);
   const uint64_t ginv = mod_pow(g, p - 2, p);
   std::vector<uint32_t> pin(M), pout(M);
@@ -939,6 +937,9 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
     flags |= PF_CFIRST_LOAD | PF_CFIRST_STORE;
   }
   const int src = *cur;
+  // every route of an axis writes N * s * O values to out_buf, which the C2R
+  // plans place in a workspace
+  b.need(out_buf, N * s * O * b.cb());
   if (N == 1) {
     Pass ps;
     ps.kind = Pass::SCALE_COPY;
@@ -984,7 +985,6 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
     return st;
   }
   const bool p2 = (N & (N - 1)) == 0;
-  b.need(out_buf, N * s * O * b.cb());
   // A long strided axis in one pass holds G*N values per CTA, so only two
   // to four adjacent columns fit: rows of 16-32 bytes, strided far apart.
   // Split into two passes of about sqrt(N), each a tile of many adjacent
@@ -999,7 +999,6 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
   }
   // four-step: n = N2*n1 + n2, k = k1 + N1*k2
   b.need(ws_buf, N * s * O * b.cb());
-  b.need(out_buf, N * s * O * b.cb());
   uint64_t N1, N2;
   if (!four_step_split(b, N, &N1, &N2))
     return fail(B2F_ERR_UNSUPPORTED_LENGTH,
