@@ -10,7 +10,6 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
-#include <type_traits>
 
 #include "dft_consts.h"
 
@@ -149,40 +148,6 @@ FFT_D cpx<S> czero() {
 template <class S>
 FFT_D cpx<S> cfrom(double re, double im) {
   return {Scalar<S>::from_double(re), Scalar<S>::from_double(im)};
-}
-
-// A value of a 16-byte buffer whose storage type is IO, computed on as S.
-// IO = S: the value itself.  IO = df with S = double (the df64 plans compute
-// in native f64, 53 bits against the 44-48 of the hi + lo pair): a buffer
-// that holds df64 words (words = true: the caller's input and output) is
-// converted as it is read and written, one that holds f64 values (between
-// the passes of a plan) is not.
-template <class IO, class S>
-FFT_D cpx<S> io_in(cpx<S> raw, bool words) {
-  if constexpr (std::is_same<IO, S>::value) {
-    return raw;
-  } else {
-    if (!words) return raw;
-    auto join = [](double w) {
-      return (double)__int_as_float(__double2loint(w)) + (double)__int_as_float(__double2hiint(w));
-    };
-    return {join(raw.re), join(raw.im)};
-  }
-}
-template <class IO, class S>
-FFT_D cpx<S> io_out(cpx<S> v, bool words) {
-  if constexpr (std::is_same<IO, S>::value) {
-    return v;
-  } else {
-    if (!words) return v;
-    auto split = [](double x) {
-      const float hi = __double2float_rn(x);
-      // past the f32 range (or NaN) hi is the whole value
-      const float lo = isfinite(hi) ? __double2float_rn(x - (double)hi) : 0.0f;
-      return __hiloint2double(__float_as_int(lo), __float_as_int(hi));
-    };
-    return {split(v.re), split(v.im)};
-  }
 }
 
 // Scale factor in the working type (f32 scale is computed in f32 as the

@@ -1,29 +1,25 @@
 // Precision dispatch of the kernel launchers; the kernels themselves are
 // instantiated once per precision in kernels_f32.cu, kernels_f64.cu and
-// kernels_df64.cu (compiled in parallel).  df64 plans compute in native f64
-// (a df64 product or sum takes 9 to 20 f32 operations, which made those
-// passes arithmetic-bound: 16 lines of 2^20 points took 1.159 ms, 0.361 ms
-// as f64 kernels that convert the words at the ends of a plan, against
-// 0.344 ms for the f64 plan; error against 64 bits 6.7e-15 -> 8.5e-16).
+// kernels_df64.cu (compiled in parallel).
 #include <mutex>
 
 #include "kernels.h"
 
 namespace b2f {
 
-template <class S, class IO = S>
+template <class S>
 cudaError_t launch_lines_t(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
-template <class S, class IO = S>
+template <class S>
 cudaError_t launch_rader_t(const RaderParams&, unsigned, unsigned, size_t, cudaStream_t);
-template <class S, class IO = S>
+template <class S>
 cudaError_t launch_bluestein_t(const BluesteinParams&, unsigned, unsigned, size_t, cudaStream_t);
 template <class S>
 cudaError_t launch_r2c_t(const RealParams&, unsigned, unsigned, size_t, cudaStream_t);
 template <class S>
 cudaError_t launch_c2r_t(const RealParams&, unsigned, unsigned, size_t, cudaStream_t);
-template <class S, class IO = S>
-cudaError_t launch_scale_copy_t(const void*, void*, uint64_t, double, bool, uint32_t, cudaStream_t);
-template <class S, class IO = S>
+template <class S>
+cudaError_t launch_scale_copy_t(const void*, void*, uint64_t, double, bool, cudaStream_t);
+template <class S>
 cudaError_t launch_blue_elem_t(const BlueElemParams&, cudaStream_t);
 
 template <class S>
@@ -49,7 +45,7 @@ cudaError_t launch_blue_elem(Prec p, const BlueElemParams& prm, cudaStream_t st)
   switch (p) {
     case PREC_F32: return launch_blue_elem_t<float>(prm, st);
     case PREC_F64: return launch_blue_elem_t<double>(prm, st);
-    case PREC_DF64: return launch_blue_elem_t<double, df>(prm, st);
+    case PREC_DF64: return launch_blue_elem_t<df>(prm, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -68,7 +64,7 @@ size_t max_smem_per_block() {
   return g_max_smem;
 }
 
-template <class S, int E, bool COLMAJOR, class IO = S>
+template <class S, int E, bool COLMAJOR>
 cudaError_t launch_pow2_t(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
 
 cudaError_t launch_pow2_fixed(Prec prec, int E, bool colmajor, const LinesParams& prm,
@@ -112,8 +108,8 @@ cudaError_t launch_pow2(Prec p, int E, bool colmajor, const LinesParams& prm, un
       return colmajor ? launch_pow2_t<double, 16, true>(prm, grid, threads, smem, st)
                       : launch_pow2_t<double, 16, false>(prm, grid, threads, smem, st);
     case PREC_DF64:
-      return colmajor ? launch_pow2_t<double, 16, true, df>(prm, grid, threads, smem, st)
-                      : launch_pow2_t<double, 16, false, df>(prm, grid, threads, smem, st);
+      return colmajor ? launch_pow2_t<df, 16, true>(prm, grid, threads, smem, st)
+                      : launch_pow2_t<df, 16, false>(prm, grid, threads, smem, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -123,7 +119,7 @@ cudaError_t launch_lines(Prec p, const LinesParams& prm, unsigned grid, unsigned
   switch (p) {
     case PREC_F32: return launch_lines_t<float>(prm, grid, threads, smem, st);
     case PREC_F64: return launch_lines_t<double>(prm, grid, threads, smem, st);
-    case PREC_DF64: return launch_lines_t<double, df>(prm, grid, threads, smem, st);
+    case PREC_DF64: return launch_lines_t<df>(prm, grid, threads, smem, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -133,7 +129,7 @@ cudaError_t launch_rader(Prec p, const RaderParams& prm, unsigned grid, unsigned
   switch (p) {
     case PREC_F32: return launch_rader_t<float>(prm, grid, threads, smem, st);
     case PREC_F64: return launch_rader_t<double>(prm, grid, threads, smem, st);
-    case PREC_DF64: return launch_rader_t<double, df>(prm, grid, threads, smem, st);
+    case PREC_DF64: return launch_rader_t<df>(prm, grid, threads, smem, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -143,7 +139,7 @@ cudaError_t launch_bluestein(Prec p, const BluesteinParams& prm, unsigned grid,
   switch (p) {
     case PREC_F32: return launch_bluestein_t<float>(prm, grid, threads, smem, st);
     case PREC_F64: return launch_bluestein_t<double>(prm, grid, threads, smem, st);
-    case PREC_DF64: return launch_bluestein_t<double, df>(prm, grid, threads, smem, st);
+    case PREC_DF64: return launch_bluestein_t<df>(prm, grid, threads, smem, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -167,15 +163,11 @@ cudaError_t launch_c2r(Prec p, const RealParams& prm, unsigned grid, unsigned th
 }
 
 cudaError_t launch_scale_copy(Prec p, const void* in, void* out, uint64_t n, double scale,
-                              bool conj, uint32_t flags, cudaStream_t st) {
+                              bool conj, cudaStream_t st) {
   switch (p) {
-    case PREC_F32: return launch_scale_copy_t<float>(in, out, n, scale, conj, 0, st);
-    case PREC_F64: return launch_scale_copy_t<double>(in, out, n, scale, conj, 0, st);
-    case PREC_DF64:
-      // words to words: df64 arithmetic, which keeps a low word of any size
-      if ((flags & PF_DF_IN) && (flags & PF_DF_OUT))
-        return launch_scale_copy_t<df>(in, out, n, scale, conj, 0, st);
-      return launch_scale_copy_t<double, df>(in, out, n, scale, conj, flags, st);
+    case PREC_F32: return launch_scale_copy_t<float>(in, out, n, scale, conj, st);
+    case PREC_F64: return launch_scale_copy_t<double>(in, out, n, scale, conj, st);
+    case PREC_DF64: return launch_scale_copy_t<df>(in, out, n, scale, conj, st);
   }
   return cudaErrorInvalidValue;
 }

@@ -22,8 +22,6 @@ enum PassFlags : uint32_t {
   PF_CFIRST_STORE = 1u << 5, // adjacent lines first when storing
   PF_TW_TABLE = 1u << 6,     // stage twiddles from the plan table (else computed)
   PF_STORE_SMEM = 1u << 7,   // register kernel: final store through shared memory, lines first
-  PF_DF_IN = 1u << 8,        // df64 plan: the input buffer holds df64 words (else f64 values)
-  PF_DF_OUT = 1u << 9,       // df64 plan: the output buffer holds df64 words
 };
 
 // Where the G lines of one CTA live.  Lines are numbered
@@ -179,9 +177,8 @@ cudaError_t launch_real_elem(Prec p, const RealElemParams& prm, cudaStream_t st)
 cudaError_t launch_small_volume(Prec p, const SmallVolumeParams& prm, unsigned threads,
                                 size_t smem, cudaStream_t st);
 // out[i] = scale * (conj?) in[i] for n complex values (length-1 transforms).
-// flags: PF_DF_IN / PF_DF_OUT of a df64 plan.
 cudaError_t launch_scale_copy(Prec p, const void* in, void* out, uint64_t n, double scale,
-                              bool conj, uint32_t flags, cudaStream_t st);
+                              bool conj, cudaStream_t st);
 
 // Largest dynamic shared memory a CTA may use on this device.
 size_t max_smem_per_block();

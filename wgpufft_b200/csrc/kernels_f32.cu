@@ -3,22 +3,22 @@
 #include "regfft.cuh"
 
 namespace b2f {
-template cudaError_t launch_lines_t<float, float>(const LinesParams&, unsigned, unsigned, size_t,
+template cudaError_t launch_lines_t<float>(const LinesParams&, unsigned, unsigned, size_t,
                                               cudaStream_t);
-template cudaError_t launch_rader_t<float, float>(const RaderParams&, unsigned, unsigned, size_t,
+template cudaError_t launch_rader_t<float>(const RaderParams&, unsigned, unsigned, size_t,
                                               cudaStream_t);
-template cudaError_t launch_bluestein_t<float, float>(const BluesteinParams&, unsigned, unsigned,
+template cudaError_t launch_bluestein_t<float>(const BluesteinParams&, unsigned, unsigned,
                                                   size_t, cudaStream_t);
-template cudaError_t launch_scale_copy_t<float, float>(const void*, void*, uint64_t, double, bool,
-                                             uint32_t, cudaStream_t);
+template cudaError_t launch_scale_copy_t<float>(const void*, void*, uint64_t, double, bool,
+                                             cudaStream_t);
 template cudaError_t launch_r2c_t<float>(const RealParams&, unsigned, unsigned, size_t,
                                             cudaStream_t);
 template cudaError_t launch_c2r_t<float>(const RealParams&, unsigned, unsigned, size_t,
                                             cudaStream_t);
-template cudaError_t launch_blue_elem_t<float, float>(const BlueElemParams&, cudaStream_t);
-template cudaError_t launch_pow2_t<float, 16, false, float>(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
-template cudaError_t launch_pow2_t<float, 16, true, float>(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
-template cudaError_t launch_pow2_t<float, 32, true, float>(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
+template cudaError_t launch_blue_elem_t<float>(const BlueElemParams&, cudaStream_t);
+template cudaError_t launch_pow2_t<float, 16, false>(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
+template cudaError_t launch_pow2_t<float, 16, true>(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
+template cudaError_t launch_pow2_t<float, 32, true>(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
 template cudaError_t launch_real_elem_t<float>(const RealElemParams&, cudaStream_t);
 template cudaError_t launch_small_volume_t<float>(const SmallVolumeParams&, unsigned, size_t,
                                                   cudaStream_t);

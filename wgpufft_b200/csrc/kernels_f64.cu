@@ -3,20 +3,20 @@
 #include "regfft.cuh"
 
 namespace b2f {
-template cudaError_t launch_lines_t<double, double>(const LinesParams&, unsigned, unsigned, size_t,
+template cudaError_t launch_lines_t<double>(const LinesParams&, unsigned, unsigned, size_t,
                                               cudaStream_t);
-template cudaError_t launch_rader_t<double, double>(const RaderParams&, unsigned, unsigned, size_t,
+template cudaError_t launch_rader_t<double>(const RaderParams&, unsigned, unsigned, size_t,
                                               cudaStream_t);
-template cudaError_t launch_bluestein_t<double, double>(const BluesteinParams&, unsigned, unsigned,
+template cudaError_t launch_bluestein_t<double>(const BluesteinParams&, unsigned, unsigned,
                                                   size_t, cudaStream_t);
-template cudaError_t launch_scale_copy_t<double, double>(const void*, void*, uint64_t, double, bool,
-                                             uint32_t, cudaStream_t);
+template cudaError_t launch_scale_copy_t<double>(const void*, void*, uint64_t, double, bool,
+                                             cudaStream_t);
 template cudaError_t launch_r2c_t<double>(const RealParams&, unsigned, unsigned, size_t,
                                             cudaStream_t);
 template cudaError_t launch_c2r_t<double>(const RealParams&, unsigned, unsigned, size_t,
                                             cudaStream_t);
-template cudaError_t launch_blue_elem_t<double, double>(const BlueElemParams&, cudaStream_t);
-template cudaError_t launch_pow2_t<double, 16, false, double>(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
-template cudaError_t launch_pow2_t<double, 16, true, double>(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
+template cudaError_t launch_blue_elem_t<double>(const BlueElemParams&, cudaStream_t);
+template cudaError_t launch_pow2_t<double, 16, false>(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
+template cudaError_t launch_pow2_t<double, 16, true>(const LinesParams&, unsigned, unsigned, size_t, cudaStream_t);
 template cudaError_t launch_real_elem_t<double>(const RealElemParams&, cudaStream_t);
 }  // namespace b2f

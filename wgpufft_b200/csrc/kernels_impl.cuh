@@ -114,12 +114,11 @@ FFT_D bool fixed_line_walk(uint32_t G, uint32_t T) {
   return (G & (G - 1)) == 0 && (T & (G - 1)) == 0;
 }
 
-template <class S, class IO = S>
+template <class S>
 FFT_D void load_lines(C<S>* sm, const LinesParams& p, const Group& g, uint32_t tid, uint32_t T) {
   constexpr int PAD = PadOf<S>::value;
   const C<S>* __restrict__ in = (const C<S>*)p.in;
   const bool conj_in = p.flags & PF_CONJ_IN;
-  const bool words = p.flags & PF_DF_IN;
   if ((p.flags & PF_CFIRST_LOAD) && fixed_line_walk(p.G, T)) {
     const uint32_t lg = 31 - __clz(p.G), c = tid & (p.G - 1), dn = T >> lg;
     if (c < g.nvalid) {
@@ -134,13 +133,12 @@ FFT_D void load_lines(C<S>* sm, const LinesParams& p, const Group& g, uint32_t t
         for (int u = 0; u < U; ++u) v[u] = src[(int64_t)(n + u * dn) * es];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          v[u] = io_in<IO>(v[u], words);
           if (conj_in) v[u].im = -v[u].im;
           line[pidx<PAD>(n + u * dn)] = v[u];
         }
       }
       for (; n < p.N; n += dn) {
-        C<S> v = io_in<IO>(src[(int64_t)n * es], words);
+        C<S> v = src[(int64_t)n * es];
         if (conj_in) v.im = -v.im;
         line[pidx<PAD>(n)] = v;
       }
@@ -155,20 +153,18 @@ FFT_D void load_lines(C<S>* sm, const LinesParams& p, const Group& g, uint32_t t
       },
       [&](uint32_t c, uint32_t n, C<S> v) {
         if (c < g.nvalid) {
-          v = io_in<IO>(v, words);
           if (conj_in) v.im = -v.im;
           sm[c * p.LD + pidx<PAD>(n)] = v;
         }
       });
 }
 
-template <class S, class IO = S>
+template <class S>
 FFT_D void store_lines(const C<S>* sm, const LinesParams& p, const Group& g, uint32_t tid,
                        uint32_t T) {
   constexpr int PAD = PadOf<S>::value;
   C<S>* __restrict__ out = (C<S>*)p.out;
   const uint32_t fl = p.flags;
-  const bool words = fl & PF_DF_OUT;
   const S sc = Scalar<S>::from_double(p.scale);
   if ((fl & PF_CFIRST_STORE) && fixed_line_walk(p.G, T)) {
     const uint32_t lg = 31 - __clz(p.G), c = tid & (p.G - 1), dn = T >> lg;
@@ -195,7 +191,7 @@ FFT_D void store_lines(const C<S>* sm, const LinesParams& p, const Group& g, uin
     auto put = [&](uint32_t n, C<S> v) {
       if (fl & PF_SCALE) v = cscale(v, sc);
       if (fl & PF_CONJ_OUT) v.im = -v.im;
-      dst[(int64_t)n * es] = io_out<IO>(v, words);
+      dst[(int64_t)n * es] = v;
     };
     uint32_t n = n0;
     if (fl & PF_TW_STORE) {
@@ -236,7 +232,7 @@ FFT_D void store_lines(const C<S>* sm, const LinesParams& p, const Group& g, uin
             C<S> v = cmul(sm[c * p.LD + pidx<PAD>(n)], w);
             if (fl & PF_SCALE) v = cscale(v, sc);
             if (fl & PF_CONJ_OUT) v.im = -v.im;
-            out[g.out0 + (int64_t)c * g.dl_out + (int64_t)n * p.io.out_es] = io_out<IO>(v, words);
+            out[g.out0 + (int64_t)c * g.dl_out + (int64_t)n * p.io.out_es] = v;
           }
         });
     return;
@@ -246,7 +242,7 @@ FFT_D void store_lines(const C<S>* sm, const LinesParams& p, const Group& g, uin
       C<S> v = sm[c * p.LD + pidx<PAD>(n)];
       if (fl & PF_SCALE) v = cscale(v, sc);
       if (fl & PF_CONJ_OUT) v.im = -v.im;
-      out[g.out0 + (int64_t)c * g.dl_out + (int64_t)n * p.io.out_es] = io_out<IO>(v, words);
+      out[g.out0 + (int64_t)c * g.dl_out + (int64_t)n * p.io.out_es] = v;
     }
   });
 }
@@ -258,17 +254,17 @@ FFT_D const C<S>* tw_of(const LinesParams& p) {
 
 // ------------------------------------------------------------ mixed radix
 // Shared memory: two line buffers of G*LD elements (ping-pong).
-template <class S, class IO = S>
+template <class S>
 __global__ void __launch_bounds__(512) k_lines(const __grid_constant__ LinesParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C<S>* A = reinterpret_cast<C<S>*>(smem_raw);
   C<S>* B = A + p.G * p.LD;
   const uint32_t tid = threadIdx.x, T = blockDim.x;
   const Group g = group_of(p.io, p.G, blockIdx.x);
-  load_lines<S, IO>(A, p, g, tid, T);
+  load_lines<S>(A, p, g, tid, T);
   __syncthreads();
   const C<S>* res = fft_lines_smem<S>(A, B, p.sch, p.G, p.LD, tid, T, tw_of<S>(p));
-  store_lines<S, IO>(res, p, g, tid, T);
+  store_lines<S>(res, p, g, tid, T);
 }
 
 // ------------------------------------------------------------------ Rader
@@ -277,7 +273,7 @@ __global__ void __launch_bounds__(512) k_lines(const __grid_constant__ LinesPara
 // FFT_{p-1}, the product with the precomputed spectrum of b, and the
 // inverse FFT (src/runtime/rader_axis.rs:1228-1336 builds the same pieces).
 // Shared memory: two buffers of G*LD, then x0[G] and X0[G].
-template <class S, class IO = S>
+template <class S>
 __global__ void __launch_bounds__(512) k_rader(const __grid_constant__ RaderParams rp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int PAD = PadOf<S>::value;
@@ -289,7 +285,7 @@ __global__ void __launch_bounds__(512) k_rader(const __grid_constant__ RaderPara
   const uint32_t tid = threadIdx.x, T = blockDim.x;
   const uint32_t P = p.N, P1 = P - 1, G = p.G, LD = p.LD;
   const Group g = group_of(p.io, G, blockIdx.x);
-  load_lines<S, IO>(A, p, g, tid, T);
+  load_lines<S>(A, p, g, tid, T);
   __syncthreads();
   if (tid < G) x0s[tid] = A[tid * LD];
   for_each_elem_batched<8, uint32_t>(
@@ -331,7 +327,7 @@ __global__ void __launch_bounds__(512) k_rader(const __grid_constant__ RaderPara
           }
           if (fl & PF_SCALE) v = cscale(v, sc);
           if (fl & PF_CONJ_OUT) v.im = -v.im;
-          out[g.out0 + (int64_t)c * g.dl_out + (int64_t)n * p.io.out_es] = io_out<IO>(v, fl & PF_DF_OUT);
+          out[g.out0 + (int64_t)c * g.dl_out + (int64_t)n * p.io.out_es] = v;
         }
       });
 }
@@ -347,7 +343,7 @@ FFT_D C<S> chirp(uint64_t n, uint32_t N) {
   return twiddle<S>((n * n) % twoN, twoN);
 }
 
-template <class S, class IO = S>
+template <class S>
 __global__ void __launch_bounds__(512) k_bluestein(const __grid_constant__ BluesteinParams bp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int PAD = PadOf<S>::value;
@@ -361,7 +357,6 @@ __global__ void __launch_bounds__(512) k_bluestein(const __grid_constant__ Blues
   {
     const C<S>* __restrict__ in = (const C<S>*)p.in;
     const bool conj_in = p.flags & PF_CONJ_IN;
-    const bool words = p.flags & PF_DF_IN;
     for_each_elem_batched<BatchU<S>::value, CPair<S>>(
         N, p.dN, G, p.dG, p.flags & PF_CFIRST_LOAD, tid, T,
         [&](uint32_t c, uint32_t n) {
@@ -374,7 +369,6 @@ __global__ void __launch_bounds__(512) k_bluestein(const __grid_constant__ Blues
         },
         [&](uint32_t c, uint32_t n, CPair<S> x) {
           if (c < g.nvalid) {
-            x.a = io_in<IO>(x.a, words);
             if (conj_in) x.a.im = -x.a.im;
             A[c * LD + pidx<PAD>(n)] = cmul(x.a, x.b);
           }
@@ -416,7 +410,7 @@ __global__ void __launch_bounds__(512) k_bluestein(const __grid_constant__ Blues
           C<S> v = cmul(w, ch);
           if (fl & PF_SCALE) v = cscale(v, sc);
           if (fl & PF_CONJ_OUT) v.im = -v.im;
-          out[g.out0 + (int64_t)c * g.dl_out + (int64_t)k * p.io.out_es] = io_out<IO>(v, fl & PF_DF_OUT);
+          out[g.out0 + (int64_t)c * g.dl_out + (int64_t)k * p.io.out_es] = v;
         }
       });
 }
@@ -596,11 +590,10 @@ __global__ void __launch_bounds__(512) k_c2r_odd(const __grid_constant__ RealPar
 // the whole grid and many short lines share it alike.
 constexpr uint32_t kElemChunk = 2048;
 
-template <class S, class IO = S>
+template <class S>
 __global__ void __launch_bounds__(256) k_blue_elem(const __grid_constant__ BlueElemParams p) {
   const uint32_t tid = threadIdx.x, T = blockDim.x;
   const uint32_t N = p.N, M = p.M;
-  const bool win = p.flags & PF_DF_IN, wout = p.flags & PF_DF_OUT;
   const S sc = Scalar<S>::from_double(p.scale);
   const C<S>* __restrict__ ctab = (const C<S>*)p.chirp;
   // points per line this pass writes
@@ -618,7 +611,7 @@ __global__ void __launch_bounds__(256) k_blue_elem(const __grid_constant__ BlueE
       for (uint32_t m = c0 + tid; m < c1; m += T) {
         C<S> v = czero<S>();
         if (m < N) {
-          v = io_in<IO>(in[base + (int64_t)m * (int64_t)p.s], win);
+          v = in[base + (int64_t)m * (int64_t)p.s];
           if (p.flags & PF_CONJ_IN) v.im = -v.im;
           v = cmul(v, ctab ? ctab[m] : chirp<S>(m, N));
         }
@@ -637,12 +630,12 @@ __global__ void __launch_bounds__(256) k_blue_elem(const __grid_constant__ BlueE
       const C<S>* __restrict__ in = (const C<S>*)p.in;
       C<S>* __restrict__ ws = (C<S>*)p.out + l * M;
       for (uint32_t q = c0 + tid; q < c1; q += T) {
-        C<S> v = io_in<IO>(in[base + (int64_t)p.perm_in[q] * (int64_t)p.s], win);
+        C<S> v = in[base + (int64_t)p.perm_in[q] * (int64_t)p.s];
         if (p.flags & PF_CONJ_IN) v.im = -v.im;
         ws[q] = v;
       }
       if (c0 == 0 && tid == 0) {
-        C<S> v = io_in<IO>(in[base], win);
+        C<S> v = in[base];
         if (p.flags & PF_CONJ_IN) v.im = -v.im;
         ((C<S>*)p.x0)[2 * l] = v;
       }
@@ -673,7 +666,7 @@ __global__ void __launch_bounds__(256) k_blue_elem(const __grid_constant__ BlueE
         }
         if (p.flags & PF_SCALE) v = cscale(v, sc);
         if (p.flags & PF_CONJ_OUT) v.im = -v.im;
-        out[base + (int64_t)n * (int64_t)p.s] = io_out<IO>(v, wout);
+        out[base + (int64_t)n * (int64_t)p.s] = v;
       }
     } else {
       const C<S>* __restrict__ ws = (const C<S>*)p.in + l * M;
@@ -684,7 +677,7 @@ __global__ void __launch_bounds__(256) k_blue_elem(const __grid_constant__ BlueE
         C<S> v = cmul(w, ctab ? ctab[k] : chirp<S>(k, N));
         if (p.flags & PF_SCALE) v = cscale(v, sc);
         if (p.flags & PF_CONJ_OUT) v.im = -v.im;
-        out[base + (int64_t)k * (int64_t)p.s] = io_out<IO>(v, wout);
+        out[base + (int64_t)k * (int64_t)p.s] = v;
       }
     }
   }
@@ -725,15 +718,15 @@ __global__ void __launch_bounds__(256) k_real_elem(const __grid_constant__ RealE
   }
 }
 
-template <class S, class IO = S>
+template <class S>
 __global__ void k_scale_copy(const C<S>* __restrict__ in, C<S>* __restrict__ out, uint64_t n,
-                             double scale, int conj_flag, uint32_t flags) {
+                             double scale, int conj_flag) {
   const S sc = Scalar<S>::from_double(scale);
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
-    C<S> v = cscale(io_in<IO>(in[i], flags & PF_DF_IN), sc);
+    C<S> v = cscale(in[i], sc);
     if (conj_flag) v.im = -v.im;
-    out[i] = io_out<IO>(v, flags & PF_DF_OUT);
+    out[i] = v;
   }
 }
 
@@ -823,20 +816,20 @@ cudaError_t launch_small_volume_t(const SmallVolumeParams& prm, unsigned threads
                                   cudaStream_t st) {
   return launch(k_small_volume<S>, prm, (unsigned)prm.nvol, threads, smem, st);
 }
-template <class S, class IO>
+template <class S>
 cudaError_t launch_lines_t(const LinesParams& prm, unsigned grid, unsigned threads, size_t smem,
                            cudaStream_t st) {
-  return launch(k_lines<S, IO>, prm, grid, threads, smem, st);
+  return launch(k_lines<S>, prm, grid, threads, smem, st);
 }
-template <class S, class IO>
+template <class S>
 cudaError_t launch_rader_t(const RaderParams& prm, unsigned grid, unsigned threads, size_t smem,
                            cudaStream_t st) {
-  return launch(k_rader<S, IO>, prm, grid, threads, smem, st);
+  return launch(k_rader<S>, prm, grid, threads, smem, st);
 }
-template <class S, class IO>
+template <class S>
 cudaError_t launch_bluestein_t(const BluesteinParams& prm, unsigned grid, unsigned threads,
                                size_t smem, cudaStream_t st) {
-  return launch(k_bluestein<S, IO>, prm, grid, threads, smem, st);
+  return launch(k_bluestein<S>, prm, grid, threads, smem, st);
 }
 template <class S>
 cudaError_t launch_r2c_t(const RealParams& prm, unsigned grid, unsigned threads, size_t smem,
@@ -850,13 +843,13 @@ cudaError_t launch_c2r_t(const RealParams& prm, unsigned grid, unsigned threads,
   if (prm.N0 % 2 == 0) return launch(k_c2r_even<S>, prm, grid, threads, smem, st);
   return launch(k_c2r_odd<S>, prm, grid, threads, smem, st);
 }
-template <class S, class IO>
+template <class S>
 cudaError_t launch_blue_elem_t(const BlueElemParams& prm, cudaStream_t st) {
   const uint64_t L = (prm.mode == BE_POST || prm.mode == BE_RADER_POST) ? prm.N : prm.M;
   const uint64_t work = prm.nlines * ((L + kElemChunk - 1) / kElemChunk);
   uint64_t blocks = work < 148ull * 16 ? work : 148ull * 16;
   if (blocks == 0) blocks = 1;
-  k_blue_elem<S, IO><<<(unsigned)blocks, 256, 0, st>>>(prm);
+  k_blue_elem<S><<<(unsigned)blocks, 256, 0, st>>>(prm);
   return cudaGetLastError();
 }
 
@@ -870,15 +863,15 @@ cudaError_t launch_real_elem_t(const RealElemParams& prm, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-template <class S, class IO>
+template <class S>
 cudaError_t launch_scale_copy_t(const void* in, void* out, uint64_t n, double scale, bool conj,
-                                uint32_t flags, cudaStream_t st) {
+                                cudaStream_t st) {
   const unsigned threads = 256;
   uint64_t blocks = (n + threads - 1) / threads;
   if (blocks > 148ull * 32) blocks = 148ull * 32;
   if (blocks == 0) blocks = 1;
-  k_scale_copy<S, IO><<<(unsigned)blocks, threads, 0, st>>>((const C<S>*)in, (C<S>*)out, n, scale,
-                                                            conj ? 1 : 0, flags);
+  k_scale_copy<S><<<(unsigned)blocks, threads, 0, st>>>((const C<S>*)in, (C<S>*)out, n, scale,
+                                                        conj ? 1 : 0);
   return cudaGetLastError();
 }
 

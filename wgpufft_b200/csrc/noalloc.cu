@@ -68,7 +68,7 @@ static b2f_status noalloc_run(const Plan& plan, cudaStream_t st, const void* in,
         e = launch_pow2(plan.prec, p.pow2_E, p.colmajor, p.lines, p.grid, p.threads, p.smem, st);
         break;
       case Pass::SCALE_COPY:
-        e = launch_scale_copy(plan.prec, src, dst, p.copy_n, p.copy_scale, p.copy_conj, p.copy_flags, st);
+        e = launch_scale_copy(plan.prec, src, dst, p.copy_n, p.copy_scale, p.copy_conj, st);
         break;
       default:
         return fail(B2F_ERR_UNSUPPORTED_LENGTH, "route needs device tables (Rader/Bluestein)");

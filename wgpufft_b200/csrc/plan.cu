@@ -386,12 +386,24 @@ struct Builder {
         f[2 * i] = (float)v[i].real();
         f[2 * i + 1] = (float)v[i].imag();
       }
-    } else {  // f64, and df64 plans, which compute in f64
+    } else if (plan.prec == PREC_F64) {
       out.resize(v.size() * 16);
       double* d = (double*)out.data();
       for (size_t i = 0; i < v.size(); ++i) {
         d[2 * i] = v[i].real();
         d[2 * i + 1] = v[i].imag();
+      }
+    } else {
+      out.resize(v.size() * 16);
+      float* f = (float*)out.data();
+      auto split = [](double x, float* w) {
+        const float hi = (float)x;
+        w[0] = hi;
+        w[1] = std::isfinite(hi) ? (float)(x - (double)hi) : 0.0f;
+      };
+      for (size_t i = 0; i < v.size(); ++i) {
+        split(v[i].real(), f + 4 * i);
+        split(v[i].imag(), f + 4 * i + 2);
       }
     }
     return out;
@@ -1556,24 +1568,6 @@ b2f_status create_plan(const Config& cfg_in, int32_t kind, int device, Plan** ou
       if (st) return st;
     }
   }
-  for (Pass& ps : plan->passes) ps.prec = plan->prec == PREC_DF64 ? PREC_F64 : plan->prec;
-  if (plan->prec == PREC_DF64 && !plan->passes.empty()) {
-    // df64 words at the plan's two ends, f64 values between its passes
-    auto mark = [](Pass& ps, uint32_t f) {
-      ps.prec = PREC_DF64;
-      switch (ps.kind) {
-        case Pass::LINES:
-        case Pass::POW2: ps.lines.flags |= f; break;
-        case Pass::RADER: ps.rader.L.flags |= f; break;
-        case Pass::BLUESTEIN: ps.blue.L.flags |= f; break;
-        case Pass::BLUE_ELEM: ps.belem.flags |= f; break;
-        case Pass::SCALE_COPY: ps.copy_flags |= f; break;
-        default: break;  // f32 (and f64) only
-      }
-    };
-    mark(plan->passes.front(), PF_DF_IN);
-    mark(plan->passes.back(), PF_DF_OUT);
-  }
   build_diagnostics(*plan);
   if (!dry) {
     // upload tables, allocate workspaces
@@ -1637,7 +1631,7 @@ static b2f_status run_passes(const Plan& plan, cudaStream_t st, const void* in, 
       case Pass::LINES:
         p.lines.in = src;
         p.lines.out = dst;
-        e = launch_lines(p.prec, p.lines, p.grid, p.threads, p.smem, st);
+        e = launch_lines(plan.prec, p.lines, p.grid, p.threads, p.smem, st);
         break;
       case Pass::POW2: {
         p.lines.in = src;
@@ -1648,48 +1642,47 @@ static b2f_status run_passes(const Plan& plan, cudaStream_t st, const void* in, 
           done = launch_pow2_tma(p.lines, p.grid, outer, p.threads, p.tma_grid,
                                  (unsigned int*)plan.device_allocs[p.tma_err], st, &e);
         }
-        if (!done) e = launch_pow2(p.prec, p.pow2_E, p.colmajor, p.lines, p.grid, p.threads, p.smem, st);
+        if (!done) e = launch_pow2(plan.prec, p.pow2_E, p.colmajor, p.lines, p.grid, p.threads, p.smem, st);
         break;
       }
       case Pass::RADER:
         p.rader.L.in = src;
         p.rader.L.out = dst;
-        e = launch_rader(p.prec, p.rader, p.grid, p.threads, p.smem, st);
+        e = launch_rader(plan.prec, p.rader, p.grid, p.threads, p.smem, st);
         break;
       case Pass::BLUESTEIN:
         p.blue.L.in = src;
         p.blue.L.out = dst;
-        e = launch_bluestein(p.prec, p.blue, p.grid, p.threads, p.smem, st);
+        e = launch_bluestein(plan.prec, p.blue, p.grid, p.threads, p.smem, st);
         break;
       case Pass::R2C:
       case Pass::C2R:
         p.real.in = src;
         p.real.out = dst;
         if (p.real_fx)
-          e = launch_real_fixed(p.prec, p.kind == Pass::R2C, p.real, p.grid, p.threads, p.smem, st);
+          e = launch_real_fixed(plan.prec, p.kind == Pass::R2C, p.real, p.grid, p.threads, p.smem, st);
         else if (p.kind == Pass::R2C)
-          e = launch_r2c(p.prec, p.real, p.grid, p.threads, p.smem, st);
+          e = launch_r2c(plan.prec, p.real, p.grid, p.threads, p.smem, st);
         else
-          e = launch_c2r(p.prec, p.real, p.grid, p.threads, p.smem, st);
+          e = launch_c2r(plan.prec, p.real, p.grid, p.threads, p.smem, st);
         break;
       case Pass::SCALE_COPY:
-        e = launch_scale_copy(p.prec, src, dst, p.copy_n, p.copy_scale, p.copy_conj,
-                              p.copy_flags, st);
+        e = launch_scale_copy(plan.prec, src, dst, p.copy_n, p.copy_scale, p.copy_conj, st);
         break;
       case Pass::BLUE_ELEM:
         p.belem.in = src;
         p.belem.out = dst;
-        e = launch_blue_elem(p.prec, p.belem, st);
+        e = launch_blue_elem(plan.prec, p.belem, st);
         break;
       case Pass::REAL_ELEM:
         p.relem.in = src;
         p.relem.out = dst;
-        e = launch_real_elem(p.prec, p.relem, st);
+        e = launch_real_elem(plan.prec, p.relem, st);
         break;
       case Pass::SMALL_VOLUME:
         p.svol.in = src;
         p.svol.out = dst;
-        e = launch_small_volume(p.prec, p.svol, p.threads, p.smem, st);
+        e = launch_small_volume(plan.prec, p.svol, p.threads, p.smem, st);
         break;
       case Pass::TC_DFT64:
         e = launch_dft64_tc(src, dst, (const float*)plan.device_allocs[p.tc_table], p.tc_nlines,

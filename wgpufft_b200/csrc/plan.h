@@ -84,8 +84,6 @@ struct Pass {
   uint64_t copy_n = 0;
   double copy_scale = 1.0;
   bool copy_conj = false;
-  Prec prec = PREC_F32;  // arithmetic and buffers of this pass (the inner passes of a df64 plan: f64)
-  uint32_t copy_flags = 0;  // PF_DF_IN / PF_DF_OUT
   // TC_DFT64: lines, their scale and direction, device_allocs indices of the
   // operand table and of the wait-timeout flag
   uint64_t tc_nlines = 0;

@@ -5,26 +5,26 @@
 
 namespace b2f {
 
-template <class S, int E, bool COLMAJOR, int LOGN, class IO = S>
+template <class S, int E, bool COLMAJOR, int LOGN>
 inline cudaError_t fx_launch(const LinesParams& prm, unsigned grid, unsigned threads, size_t smem,
                              cudaStream_t st) {
-  return launch(k_pow2_fx<S, E, COLMAJOR, LOGN, IO>, prm, grid, threads, smem, st);
+  return launch(k_pow2_fx<S, E, COLMAJOR, LOGN>, prm, grid, threads, smem, st);
 }
 
 // f64 and df64 (16 values a thread, lines of up to 4096 points)
-template <class S, bool COLMAJOR, class IO = S>
+template <class S, bool COLMAJOR>
 inline cudaError_t fx_launch_wide(int lg, const LinesParams& prm, unsigned grid, unsigned threads,
                                   size_t smem, cudaStream_t st) {
   switch (lg) {
-    case 4: return fx_launch<S, 16, COLMAJOR, 4, IO>(prm, grid, threads, smem, st);
-    case 5: return fx_launch<S, 16, COLMAJOR, 5, IO>(prm, grid, threads, smem, st);
-    case 6: return fx_launch<S, 16, COLMAJOR, 6, IO>(prm, grid, threads, smem, st);
-    case 7: return fx_launch<S, 16, COLMAJOR, 7, IO>(prm, grid, threads, smem, st);
-    case 8: return fx_launch<S, 16, COLMAJOR, 8, IO>(prm, grid, threads, smem, st);
-    case 9: return fx_launch<S, 16, COLMAJOR, 9, IO>(prm, grid, threads, smem, st);
-    case 10: return fx_launch<S, 16, COLMAJOR, 10, IO>(prm, grid, threads, smem, st);
-    case 11: return fx_launch<S, 16, COLMAJOR, 11, IO>(prm, grid, threads, smem, st);
-    case 12: return fx_launch<S, 16, COLMAJOR, 12, IO>(prm, grid, threads, smem, st);
+    case 4: return fx_launch<S, 16, COLMAJOR, 4>(prm, grid, threads, smem, st);
+    case 5: return fx_launch<S, 16, COLMAJOR, 5>(prm, grid, threads, smem, st);
+    case 6: return fx_launch<S, 16, COLMAJOR, 6>(prm, grid, threads, smem, st);
+    case 7: return fx_launch<S, 16, COLMAJOR, 7>(prm, grid, threads, smem, st);
+    case 8: return fx_launch<S, 16, COLMAJOR, 8>(prm, grid, threads, smem, st);
+    case 9: return fx_launch<S, 16, COLMAJOR, 9>(prm, grid, threads, smem, st);
+    case 10: return fx_launch<S, 16, COLMAJOR, 10>(prm, grid, threads, smem, st);
+    case 11: return fx_launch<S, 16, COLMAJOR, 11>(prm, grid, threads, smem, st);
+    case 12: return fx_launch<S, 16, COLMAJOR, 12>(prm, grid, threads, smem, st);
     default: return cudaErrorInvalidValue;
   }
 }

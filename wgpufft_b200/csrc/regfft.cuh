@@ -100,9 +100,9 @@ FFT_D void reg_write_any(uint32_t R, const C<S> (&v)[E], C<S>* line, uint32_t t,
 }
 
 // Global load of the first stage: element (j + q*NR) of line c.
-template <class S, class IO, int R, int E>
+template <class S, int R, int E>
 FFT_D void reg_load_global(C<S> (&v)[E], const C<S>* __restrict__ in, int64_t base, int64_t es,
-                           uint32_t t, uint32_t TL, uint32_t NR, bool valid, uint32_t fl) {
+                           uint32_t t, uint32_t TL, uint32_t NR, bool valid, bool conj_in) {
   constexpr int NB = E / R;
   if (!valid) {
 #pragma unroll
@@ -115,27 +115,25 @@ FFT_D void reg_load_global(C<S> (&v)[E], const C<S>* __restrict__ in, int64_t ba
 #pragma unroll
     for (int q = 0; q < R; ++q) v[u * R + q] = in[base + (int64_t)(j + q * NR) * es];
   }
-#pragma unroll
-  for (int i = 0; i < E; ++i) v[i] = io_in<IO>(v[i], fl & PF_DF_IN);
-  if (fl & PF_CONJ_IN) {
+  if (conj_in) {
 #pragma unroll
     for (int i = 0; i < E; ++i) v[i].im = -v[i].im;
   }
 }
 
-template <class S, class IO, int E>
+template <class S, int E>
 FFT_D void reg_load_any(uint32_t R, C<S> (&v)[E], const C<S>* __restrict__ in, int64_t base,
-                        int64_t es, uint32_t t, uint32_t TL, uint32_t NR, bool valid, uint32_t fl) {
+                        int64_t es, uint32_t t, uint32_t TL, uint32_t NR, bool valid, bool cj) {
   switch (R) {
-    case 2: reg_load_global<S, IO, 2, E>(v, in, base, es, t, TL, NR, valid, fl); break;
-    case 4: reg_load_global<S, IO, 4, E>(v, in, base, es, t, TL, NR, valid, fl); break;
-    case 8: reg_load_global<S, IO, 8, E>(v, in, base, es, t, TL, NR, valid, fl); break;
-    default: reg_load_global<S, IO, 16, E>(v, in, base, es, t, TL, NR, valid, fl); break;
+    case 2: reg_load_global<S, 2, E>(v, in, base, es, t, TL, NR, valid, cj); break;
+    case 4: reg_load_global<S, 4, E>(v, in, base, es, t, TL, NR, valid, cj); break;
+    case 8: reg_load_global<S, 8, E>(v, in, base, es, t, TL, NR, valid, cj); break;
+    default: reg_load_global<S, 16, E>(v, in, base, es, t, TL, NR, valid, cj); break;
   }
 }
 
 // Last stage: output n = j + r*Ns (k = j since j < Ns) straight to HBM.
-template <class S, class IO, int R, int E>
+template <class S, int R, int E>
 FFT_D void reg_store_global(const C<S> (&v)[E], C<S>* __restrict__ out, int64_t base, int64_t es,
                             uint32_t t, uint32_t TL, uint32_t Ns, uint32_t fl, S sc,
                             uint64_t tw_row, const LinesParams& p) {
@@ -155,26 +153,26 @@ FFT_D void reg_store_global(const C<S> (&v)[E], C<S>* __restrict__ out, int64_t 
                        : twiddle<S>((tw_row * n) % p.tw_store_M, p.tw_store_M));
       if (fl & PF_SCALE) x = cscale(x, sc);
       if (fl & PF_CONJ_OUT) x.im = -x.im;
-      out[base + (int64_t)n * es] = io_out<IO>(x, fl & PF_DF_OUT);
+      out[base + (int64_t)n * es] = x;
     }
   }
 }
 
-template <class S, class IO, int E>
+template <class S, int E>
 FFT_D void reg_store_any(uint32_t R, const C<S> (&v)[E], C<S>* __restrict__ out, int64_t base,
                          int64_t es, uint32_t t, uint32_t TL, uint32_t Ns, uint32_t fl, S sc,
                          uint64_t tw_row, const LinesParams& p) {
   switch (R) {
-    case 2: reg_store_global<S, IO, 2, E>(v, out, base, es, t, TL, Ns, fl, sc, tw_row, p); break;
-    case 4: reg_store_global<S, IO, 4, E>(v, out, base, es, t, TL, Ns, fl, sc, tw_row, p); break;
-    case 8: reg_store_global<S, IO, 8, E>(v, out, base, es, t, TL, Ns, fl, sc, tw_row, p); break;
-    default: reg_store_global<S, IO, 16, E>(v, out, base, es, t, TL, Ns, fl, sc, tw_row, p); break;
+    case 2: reg_store_global<S, 2, E>(v, out, base, es, t, TL, Ns, fl, sc, tw_row, p); break;
+    case 4: reg_store_global<S, 4, E>(v, out, base, es, t, TL, Ns, fl, sc, tw_row, p); break;
+    case 8: reg_store_global<S, 8, E>(v, out, base, es, t, TL, Ns, fl, sc, tw_row, p); break;
+    default: reg_store_global<S, 16, E>(v, out, base, es, t, TL, Ns, fl, sc, tw_row, p); break;
   }
 }
 
 // G lines of N = 2^m points (E*16 >= N >= 16); blockDim = G * N / E.
 // Shared memory: G * LD elements, LD odd.
-template <class S, int E, bool COLMAJOR, class IO = S>
+template <class S, int E, bool COLMAJOR>
 __global__ void __launch_bounds__(sizeof(C<S>) == 8 ? 512 : 256)
     k_pow2(const __grid_constant__ LinesParams p) {
   constexpr int PAD = 4;
@@ -198,8 +196,8 @@ __global__ void __launch_bounds__(sizeof(C<S>) == 8 ? 512 : 256)
   const uint32_t last = sch.nst - 1;
   C<S> v[E];
   C<S>* line = sm + c * LD;
-  reg_load_any<S, IO, E>(sch.st[0].R, v, (const C<S>*)p.in, g.in0 + (int64_t)c * g.dl_in, p.io.in_es,
-                     t, TL, sch.st[0].NR, valid, p.flags);
+  reg_load_any<S, E>(sch.st[0].R, v, (const C<S>*)p.in, g.in0 + (int64_t)c * g.dl_in, p.io.in_es,
+                     t, TL, sch.st[0].NR, valid, p.flags & PF_CONJ_IN);
 #pragma unroll 1
   for (uint32_t s = 0;; ++s) {
     const StageDesc& sd = sch.st[s];
@@ -215,7 +213,7 @@ __global__ void __launch_bounds__(sizeof(C<S>) == 8 ? 512 : 256)
   if (!(p.flags & PF_STORE_SMEM)) {
     if (valid) {
       const uint64_t row = (p.flags & PF_TW_STORE) ? fdiv((uint32_t)(g.c0 + c), p.d_tw) : 0;
-      reg_store_any<S, IO, E>(sl.R, v, (C<S>*)p.out, g.out0 + (int64_t)c * g.dl_out, p.io.out_es, t,
+      reg_store_any<S, E>(sl.R, v, (C<S>*)p.out, g.out0 + (int64_t)c * g.dl_out, p.io.out_es, t,
                           TL, sl.Ns, p.flags, sc, row, p);
     }
     return;
@@ -237,15 +235,15 @@ __global__ void __launch_bounds__(sizeof(C<S>) == 8 ? 512 : 256)
       }
       if (fl & PF_SCALE) x = cscale(x, sc);
       if (fl & PF_CONJ_OUT) x.im = -x.im;
-      out[g.out0 + (int64_t)cc * g.dl_out + (int64_t)n * p.io.out_es] = io_out<IO>(x, fl & PF_DF_OUT);
+      out[g.out0 + (int64_t)cc * g.dl_out + (int64_t)n * p.io.out_es] = x;
     }
   });
 }
 
-template <class S, int E, bool COLMAJOR, class IO>
+template <class S, int E, bool COLMAJOR>
 cudaError_t launch_pow2_t(const LinesParams& prm, unsigned grid, unsigned threads, size_t smem,
                           cudaStream_t st) {
-  return launch(k_pow2<S, E, COLMAJOR, IO>, prm, grid, threads, smem, st);
+  return launch(k_pow2<S, E, COLMAJOR>, prm, grid, threads, smem, st);
 }
 
 }  // namespace b2f

@@ -123,7 +123,7 @@ struct FxBounds {
   static constexpr int threads = wide || (COLMAJOR && E == 16) ? 256 : 512;
   static constexpr int blocks = wide ? 2 : (COLMAJOR ? (E == 16 ? 3 : 1) : 2);
 };
-template <class S, int E, bool COLMAJOR, int LOGN, class IO = S>
+template <class S, int E, bool COLMAJOR, int LOGN>
 __global__ void __launch_bounds__(FxBounds<S, E, COLMAJOR>::threads, FxBounds<S, E, COLMAJOR>::blocks)
     k_pow2_fx(const __grid_constant__ LinesParams p) {
   using P = P2Sched<LOGN>;
@@ -157,8 +157,6 @@ __global__ void __launch_bounds__(FxBounds<S, E, COLMAJOR>::threads, FxBounds<S,
 #pragma unroll
       for (int q = 0; q < R0; ++q) v[u * R0 + q] = b[(int64_t)q * NR0 * es];
     }
-#pragma unroll
-    for (int i = 0; i < E; ++i) v[i] = io_in<IO>(v[i], p.flags & PF_DF_IN);
     if (p.flags & PF_CONJ_IN) {
 #pragma unroll
       for (int i = 0; i < E; ++i) v[i].im = -v[i].im;
@@ -203,7 +201,7 @@ __global__ void __launch_bounds__(FxBounds<S, E, COLMAJOR>::threads, FxBounds<S,
         }
         if (fl & PF_SCALE) x = cscale(x, sc);
         if (fl & PF_CONJ_OUT) x.im = -x.im;
-        b[(int64_t)r * NSL * es] = io_out<IO>(x, fl & PF_DF_OUT);
+        b[(int64_t)r * NSL * es] = x;
       }
     }
     return;
@@ -230,7 +228,7 @@ __global__ void __launch_bounds__(FxBounds<S, E, COLMAJOR>::threads, FxBounds<S,
       }
       if (fl & PF_SCALE) x = cscale(x, sc);
       if (fl & PF_CONJ_OUT) x.im = -x.im;
-      out[g.out0 + (int64_t)cc * g.dl_out + (int64_t)n * p.io.out_es] = io_out<IO>(x, fl & PF_DF_OUT);
+      out[g.out0 + (int64_t)cc * g.dl_out + (int64_t)n * p.io.out_es] = x;
     }
   });
 }

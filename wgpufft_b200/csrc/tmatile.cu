@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(256, 3)
     if (valid) {
       const StageDesc& sl = sch.st[last];
       const uint64_t row = (p.flags & PF_TW_STORE) ? fdiv((uint32_t)(g.c0 + c), p.d_tw) : 0;
-      reg_store_any<float, float, E>(sl.R, v, (C*)p.out, g.out0 + (int64_t)c * g.dl_out, p.io.out_es, t,
+      reg_store_any<float, E>(sl.R, v, (C*)p.out, g.out0 + (int64_t)c * g.dl_out, p.io.out_es, t,
                               TL, sl.Ns, p.flags, sc, row, p);
     }
   }
