@@ -8,6 +8,8 @@
 //                             and differences of x[j], x[R-j] (O(R^2/4)
 //                             multiplies), the scheme the reference uses for
 //                             its odd radices (src/runtime/axis_plan.rs:3079);
+//   R = 6, 10, 12, 14, 15   : two coprime factors, the prime-factor mapping (no
+//                             twiddles between them, only renamed registers);
 //   R = 9, 16              : two nested codelets R = A*B with the
 //                             W_R^{n2 k1} twiddles between them as constants.
 #pragma once
@@ -134,6 +136,36 @@ struct DftComposite {
   }
 };
 
+// R = A * B, A and B coprime (Good-Thomas): input n = B*n1 + A*n2 mod R,
+// output k = k1 mod A and k2 mod B (the Chinese remainder).
+constexpr int dft_inverse_mod(int a, int m) {
+  for (int x = 1; x < m; ++x)
+    if (a * x % m == 1) return x;
+  return 1;
+}
+template <class S, int A, int B>
+struct DftCoprime {
+  static FFT_D void run(cpx<S>* v) {
+    constexpr int R = A * B, eA = B * dft_inverse_mod(B % A, A), eB = A * dft_inverse_mod(A % B, B);
+    cpx<S> t[R];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) {
+      cpx<S> a[A];
+#pragma unroll
+      for (int n1 = 0; n1 < A; ++n1) a[n1] = v[(B * n1 + A * n2) % R];
+      dft<S, A>(a);
+#pragma unroll
+      for (int k1 = 0; k1 < A; ++k1) t[k1 * B + n2] = a[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) {
+      dft<S, B>(t + k1 * B);
+#pragma unroll
+      for (int k2 = 0; k2 < B; ++k2) v[(eA * k1 + eB * k2) % R] = t[k1 * B + k2];
+    }
+  }
+};
+
 template <class S, int R>
 FFT_D void dft(cpx<S>* v) {
   if constexpr (R == 1) {
@@ -145,6 +177,16 @@ FFT_D void dft(cpx<S>* v) {
     Dft8<S>::run(v);
   } else if constexpr (R == 3 || R == 5 || R == 7 || R == 11 || R == 13) {
     DftOddPrime<S, R>::run(v);
+  } else if constexpr (R == 6) {
+    DftCoprime<S, 2, 3>::run(v);
+  } else if constexpr (R == 10) {
+    DftCoprime<S, 2, 5>::run(v);
+  } else if constexpr (R == 12) {
+    DftCoprime<S, 4, 3>::run(v);
+  } else if constexpr (R == 14) {
+    DftCoprime<S, 2, 7>::run(v);
+  } else if constexpr (R == 15) {
+    DftCoprime<S, 3, 5>::run(v);
   } else if constexpr (R == 9) {
     DftComposite<S, 3, 3>::run(v);
   } else if constexpr (R == 16) {

@@ -1,0 +1,11 @@
+// f32 instances of the in-place mixed-radix kernels.
+#include "ip_launch.cuh"
+
+namespace b2f {
+
+cudaError_t launch_ip_f32(IpKind kind, bool col, const IpParams& prm, unsigned grid,
+                          unsigned threads, size_t smem, cudaStream_t st) {
+  return ip_launch_t<float>(kind, col, prm, grid, threads, smem, st);
+}
+
+}  // namespace b2f

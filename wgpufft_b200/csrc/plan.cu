@@ -460,6 +460,29 @@ struct Builder {
     return true;
   }
 
+  // The in-place mixed-radix kernels (ipfft.cuh) run every smooth line they
+  // hold that has no fixed-length kernel, in f32 and f64; df64 lines, explicit
+  // launch shapes, a reversed radix order and computed twiddles stay with the
+  // ping-pong engine.
+  bool ip_on() const {
+    const Tuning& t = plan.cfg.tuning;
+    return plan.prec != PREC_DF64 && t.lines_per_block <= 0 && t.threads_per_block <= 0 &&
+           t.radix_order == 0 && t.twiddle_table;
+  }
+  // Bytes of a row line of n values in one buffer (R0 odd-pitched sub-lines)
+  // and `extra` more values.
+  size_t ip_bytes(uint64_t n, uint64_t extra = 0) const { return (n + 17 + extra) * cb(); }
+  bool fits_ip(uint64_t n, uint64_t extra = 0) const {
+    return ip_on() && n > 16 && ip_bytes(n, extra) <= smem_budget;
+  }
+  // Whether a mixed-radix line runs in one pass.
+  bool fits_lines(uint64_t n) const {
+    return fits_one_cta(n) || ((n & (n - 1)) != 0 && fits_ip(n));
+  }
+  // A Rader line of p points, a Bluestein convolution of m, in one pass.
+  bool fits_rader(uint64_t p) const { return fits_ip(p - 1, p + 2) || fits_one_cta(p); }
+  bool fits_conv(uint64_t m) const { return fits_ip(m) || fits_one_cta(m); }
+
   bool fits_one_cta(uint64_t nbuf) const { return 2 * (size_t)ld_for(nbuf) * cb() <= smem_budget; }
 
   static void fill_io_grid(LinesParams& lp, Pass& ps, uint64_t outer_n) {
@@ -474,7 +497,8 @@ struct Builder {
   // Table pointers are patched after upload, by pass index and field.
   enum Field { F_LINES_TW, F_RADER_TW, F_BLUE_TW, F_REAL_TW, F_PERM_IN, F_PERM_OUT, F_RADER_BHAT,
                F_BLUE_BHAT, F_BELEM_BHAT, F_TWS_A, F_TWS_B, F_SVOL_TW, F_BLUE_CHIRP,
-               F_BELEM_CHIRP, F_REAL_RTW, F_BELEM_PIN, F_BELEM_POUT, F_BELEM_X0 };
+               F_BELEM_CHIRP, F_REAL_RTW, F_BELEM_PIN, F_BELEM_POUT, F_BELEM_X0,
+               F_IP_TW, F_IP_PERM, F_IP_BHAT, F_IP_CHIRP, F_IP_RTW };
   struct Patch {
     size_t table, pass;
     Field field;
@@ -508,12 +532,17 @@ struct Builder {
         case F_RADER_BHAT: ps.rader.bhat = ptr; break;
         case F_BLUE_BHAT: ps.blue.bhat = ptr; break;
         case F_BELEM_BHAT: ps.belem.bhat = ptr; break;
-        case F_TWS_A: ps.lines.tws_a = ptr; break;
-        case F_TWS_B: ps.lines.tws_b = ptr; break;
+        case F_TWS_A: (ps.kind == Pass::IP ? ps.ip.tws_a : ps.lines.tws_a) = ptr; break;
+        case F_TWS_B: (ps.kind == Pass::IP ? ps.ip.tws_b : ps.lines.tws_b) = ptr; break;
         case F_SVOL_TW: ps.svol.tw = ptr; break;
         case F_BLUE_CHIRP: ps.blue.chirp = ptr; break;
         case F_BELEM_CHIRP: ps.belem.chirp = ptr; break;
         case F_REAL_RTW: ps.real.rtw = ptr; break;
+        case F_IP_TW: ps.ip.tw = ptr; break;
+        case F_IP_PERM: ps.ip.perm = (const uint32_t*)ptr; break;
+        case F_IP_BHAT: ps.ip.bhat = ptr; break;
+        case F_IP_CHIRP: ps.ip.chirp = ptr; break;
+        case F_IP_RTW: ps.ip.rtw = ptr; break;
         case F_BELEM_PIN: ps.belem.perm_in = (const uint32_t*)ptr; break;
         case F_BELEM_POUT: ps.belem.perm_out = (const uint32_t*)ptr; break;
         case F_BELEM_X0: ps.belem.x0 = const_cast<void*>(ptr); break;
@@ -584,6 +613,110 @@ static bool try_pow2_pass(Builder& b, Pass& ps, uint64_t outer_n) {
   return true;
 }
 
+// The shape of an in-place mixed-radix pass over `groups` runs of `inner_n`
+// adjacent lines, `extra` values a line beside the transform's buffer: lines
+// a CTA (G), threads, shared memory.  Returns false when one line does not
+// fit.
+static bool ip_shape(const Builder& b, Pass& ps, uint64_t inner_n, uint64_t groups,
+                     uint64_t extra) {
+  constexpr uint64_t kSms = 148;
+  IpParams& q = ps.ip;
+  const uint64_t N = q.sc.N;
+  const size_t cb = b.cb();
+  const uint64_t seg = 128 / cb;                                 // values in 128 bytes
+  const bool across = ps.ip_col || (q.flags & PF_CFIRST_STORE);  // adjacent lines share segments
+  q.pitch = ip_pitch(q.sc.NS);
+  // rows stored lines first read across the lines: an odd line pitch
+  q.LDl = q.sc.R0 * q.pitch;
+  if (!ps.ip_col && (q.flags & PF_CFIRST_STORE)) q.LDl |= 1u;
+  const size_t line = ((ps.ip_col ? N : q.LDl) + extra) * cb;
+  if (line > b.smem_budget) return false;
+  // Three CTAs of about 72 KB and 320 threads an SM (f32, 64 registers) beat
+  // seven of 32 KB: 2000-point rows 153 against 171 us over 32 M points, 360
+  // 127 against 139, 1009 (Rader) 343 against 356, though 100-point rows are
+  // 4 % better in the small ones.
+  const size_t third = 72 * 1024;
+  uint64_t G;
+  if (across) {
+    // Whole 128-byte segments where they fit at all: 1080-point columns take
+    // 54 us as one CTA of 16 lines and 1024 threads an SM, 58 as three of 8,
+    // 70 as six of 4.  A convolution's phases overlap across three CTAs
+    // instead (1009: 96 us with 4 lines in 63 KB, 105 with 8 in 126 KB), if
+    // that leaves a 32-byte sector.
+    const size_t most = ps.ip_kind == IP_LINES ? b.smem_budget : third;
+    G = seg;
+    while (G > seg / 4 && G * line > most) G >>= 1;
+    if (G == seg) G = std::max<uint64_t>(seg, third / line / seg * seg);
+    // a grid of fewer CTAs than SMs: narrower tiles
+    while (G > seg / 4 && G > 1 && (inner_n + G - 1) / G * groups < kSms) G >>= 1;
+  } else {
+    G = std::max<uint64_t>(1, third / line);
+    G = std::min<uint64_t>(G, std::max<uint64_t>(1, inner_n * groups / (3 * kSms)));
+  }
+  while (G > 1 && G * line > b.smem_budget) --G;
+  G = std::min<uint64_t>(G, std::max<uint64_t>(inner_n, 1));
+  q.G = (uint32_t)G;
+  q.lam = (uint32_t)(G * q.sc.R0);
+  q.dlam = make_fastdiv(q.lam);
+  q.dG = make_fastdiv(q.G);
+  ps.smem = G * line;
+  // the CTAs that share an SM (by shared memory and by the grid) share its
+  // threads; no more threads than the widest stage has butterflies
+  const uint64_t grid = std::max<uint64_t>(1, (inner_n + G - 1) / G * groups);
+  uint64_t ctas = std::max<uint64_t>(1, (228 * 1024) / (ps.smem + 1024));
+  ctas = std::min<uint64_t>(std::min<uint64_t>(ctas, 16), (grid + kSms - 1) / kSms);
+  uint32_t rmin = q.sc.R0 > 1 ? q.sc.R0 : 16;
+  for (uint32_t s = 0; s < q.sc.nst; ++s) rmin = std::min(rmin, q.sc.st[s].R);
+  uint64_t T = ip_threads_per_sm(b.plan.prec) / ctas / 32 * 32;
+  T = std::min<uint64_t>(T, (G * N / rmin + 31) / 32 * 32);
+  ps.threads = (unsigned)std::max<uint64_t>(T, 32);
+  return true;
+}
+
+// Starts an in-place pass: its schedule and twiddle table.
+static bool ip_begin(Builder& b, Pass& ps, IpKind kind, bool col, uint64_t N, uint64_t n,
+                     const LineIO& io, uint32_t flags, double scale) {
+  ps.kind = Pass::IP;
+  ps.ip_kind = kind;
+  ps.ip_col = col;
+  IpParams& q = ps.ip;
+  std::memset(&q, 0, sizeof(q));
+  q.io = io;
+  q.flags = flags;
+  q.scale = scale;
+  q.n = (uint32_t)n;
+  q.dn = make_fastdiv(q.n);
+  std::vector<cd> tw;
+  if (!ip_schedule(N, !col, true, b.plan.prec == PREC_F32 ? 2 : 1, q.sc, ps.radices, tw))
+    return false;
+  b.set_table(b.next_pass(), Builder::F_IP_TW, b.add_table(b.pack_complex(tw)));
+  return true;
+}
+
+static void ip_grid(Pass& ps, uint64_t outer_n) {
+  IpParams& q = ps.ip;
+  q.io.tiles = (q.io.inner_n + q.G - 1) / q.G;
+  if (q.io.tw_div == 0) q.io.tw_div = 1;
+  q.d_tw = make_fastdiv(q.io.tw_div);
+  ps.grid = (unsigned)(outer_n * q.io.mid_n * q.io.tiles);
+}
+
+// Whether the lines of an IO pattern are rows (contiguous points) or
+// columns (adjacent lines on both sides) for the in-place kernels.
+static bool ip_layout(const LineIO& io, bool* col) {
+  *col = io.in_inner == 1 && io.out_inner == 1 && io.in_es != 1;
+  return *col || io.in_es == 1;
+}
+
+// A convolution's spectrum in the order its frequencies take in the CTA.
+static std::vector<cd> ip_spectrum(const IpSched& sc, const std::vector<cd>& bvec) {
+  std::vector<cd> out(bvec.size());
+  for (uint32_t pos = 0; pos < sc.NS; ++pos)
+    for (uint32_t k0 = 0; k0 < sc.R0; ++k0)
+      out[(size_t)pos * sc.R0 + k0] = bvec[ip_frequency(sc, k0, pos)];
+  return out;
+}
+
 // One complex axis in one pass (mixed radix, line fits a CTA).
 static b2f_status add_lines_pass(Builder& b, int axis, uint64_t N, const LineIO& io,
                                  uint64_t outer_n, uint32_t flags, double scale, int src, int dst,
@@ -600,10 +733,19 @@ static b2f_status add_lines_pass(Builder& b, int axis, uint64_t N, const LineIO&
   lp.io = io;
   lp.flags = flags;
   lp.scale = scale;
+  const bool p2 = try_pow2_pass(b, ps, outer_n);
+  bool col = false;
+  if (!p2 && b.fits_ip(N) && ip_layout(io, &col)) {
+    if (!ip_begin(b, ps, IP_LINES, col, N, N, io, flags, scale) || !ip_shape(b, ps, io.inner_n, outer_n * io.mid_n, 0))
+      return fail(B2F_ERR_UNSUPPORTED_LENGTH, "UnsupportedLength { len: " + std::to_string(N) + " }");
+    ip_grid(ps, outer_n);
+    b.plan.passes.push_back(ps);
+    return B2F_OK;
+  }
   std::vector<cd> tw;
   if (!b.make_schedule(N, lp.sch, ps.radices, tw))
     return fail(B2F_ERR_UNSUPPORTED_LENGTH, "UnsupportedLength { len: " + std::to_string(N) + " }");
-  if (!try_pow2_pass(b, ps, outer_n)) {
+  if (!p2) {
     lp.LD = b.ld_for(N);
     const bool tiles = io.in_inner == 1 || io.out_inner == 1;
     if (!b.choose_launch(N, 2 * (size_t)lp.LD * b.cb(), io.inner_n, tiles && io.inner_n > 1,
@@ -642,24 +784,6 @@ static b2f_status add_rader_pass(Builder& b, int axis, uint64_t p, const LineIO&
   ps.dst = dst;
   ps.label = "rader-fused-workgroup-stage";
   ps.route = "rader";
-  RaderParams& rp = ps.rader;
-  LinesParams& lp = rp.L;
-  lp.N = (uint32_t)p;
-  lp.io = io;
-  lp.flags = flags;
-  lp.scale = scale;
-  std::vector<cd> tw;
-  if (!b.make_schedule(p - 1, lp.sch, ps.radices, tw))
-    return fail(B2F_ERR_UNSUPPORTED_LENGTH, "Rader convolution length is not smooth");
-  lp.LD = b.ld_for(p);
-  const bool tiles = io.in_inner == 1 || io.out_inner == 1;
-  if (!b.choose_launch(p - 1, 2 * (size_t)lp.LD * b.cb() + 2 * b.cb(), io.inner_n,
-                       tiles && io.inner_n > 1, &lp.G, &ps.threads))
-    return fail(B2F_ERR_UNSUPPORTED_LENGTH, "Rader line does not fit a CTA");
-  ps.smem = (2 * (size_t)lp.G * lp.LD + 2 * lp.G) * b.cb();
-  b.tw_table_for(lp.flags, tw, Builder::F_RADER_TW);
-  Builder::fill_io_grid(lp, ps, outer_n);
-  rp.dP1 = make_fastdiv((uint32_t)(p - 1));
   // tables: perm_in[q] = g^q, perm_out[n-1] = r with g^-r = n, spectrum of b
   const uint64_t g = primitive_root(p);
   const uint64_t ginv = mod_pow(g, p - 2, p);
@@ -681,6 +805,37 @@ static b2f_status add_rader_pass(Builder& b, int axis, uint64_t p, const LineIO&
   std::vector<unsigned char> bin(pin.size() * 4), bout(pout.size() * 4);
   std::memcpy(bin.data(), pin.data(), bin.size());
   std::memcpy(bout.data(), pout.data(), bout.size());
+  bool col = false;
+  // p - 1 >= 16: the in-place kernels take every Rader length
+  if (b.ip_on() && p > 16 && b.fits_rader(p) && ip_layout(io, &col) &&
+      ip_begin(b, ps, IP_RADER, col, p - 1, p, io, flags, scale) &&
+      ip_shape(b, ps, io.inner_n, outer_n * io.mid_n, p + 2)) {
+    ip_grid(ps, outer_n);
+    b.set_table(b.next_pass(), Builder::F_IP_PERM, b.add_table(std::move(bin)));
+    b.set_table(b.next_pass(), Builder::F_IP_BHAT,
+                b.add_table(b.pack_complex(ip_spectrum(ps.ip.sc, bvec))));
+    b.plan.passes.push_back(ps);
+    return B2F_OK;
+  }
+  ps.kind = Pass::RADER;
+  RaderParams& rp = ps.rader;
+  LinesParams& lp = rp.L;
+  lp.N = (uint32_t)p;
+  lp.io = io;
+  lp.flags = flags;
+  lp.scale = scale;
+  std::vector<cd> tw;
+  if (!b.make_schedule(p - 1, lp.sch, ps.radices, tw))
+    return fail(B2F_ERR_UNSUPPORTED_LENGTH, "Rader convolution length is not smooth");
+  lp.LD = b.ld_for(p);
+  const bool tiles = io.in_inner == 1 || io.out_inner == 1;
+  if (!b.choose_launch(p - 1, 2 * (size_t)lp.LD * b.cb() + 2 * b.cb(), io.inner_n,
+                       tiles && io.inner_n > 1, &lp.G, &ps.threads))
+    return fail(B2F_ERR_UNSUPPORTED_LENGTH, "Rader line does not fit a CTA");
+  ps.smem = (2 * (size_t)lp.G * lp.LD + 2 * lp.G) * b.cb();
+  b.tw_table_for(lp.flags, tw, Builder::F_RADER_TW);
+  Builder::fill_io_grid(lp, ps, outer_n);
+  rp.dP1 = make_fastdiv((uint32_t)(p - 1));
   b.set_table(b.next_pass(), Builder::F_PERM_IN, b.add_table(std::move(bin)));
   b.set_table(b.next_pass(), Builder::F_PERM_OUT, b.add_table(std::move(bout)));
   b.set_table(b.next_pass(), Builder::F_RADER_BHAT, b.add_table(b.pack_complex(bvec)));
@@ -714,15 +869,16 @@ static double stage_cost(uint32_t R) {
 static uint64_t bluestein_length(const Builder& b, uint64_t n) {
   uint64_t m0 = 2 * n - 1;
   while (!is_smooth7(m0)) ++m0;
-  if (!b.fits_one_cta(m0)) return m0;
-  auto cost = [](uint64_t m) {
+  if (!b.fits_conv(m0)) return m0;
+  auto cost = [&](uint64_t m) {
+    if (b.fits_ip(m)) return ip_cost(ip_radices(m, 2)) * (double)m;
     double c = 0;
     for (uint32_t R : stage_radices(m)) c += stage_cost(R);
     return c * (double)m;
   };
   uint64_t best = m0;
   double best_c = cost(m0);
-  for (uint64_t m = m0 + 1; m <= 9 * n / 4 && b.fits_one_cta(m); ++m) {
+  for (uint64_t m = m0 + 1; m <= 9 * n / 4 && b.fits_conv(m); ++m) {
     if (!is_smooth7(m)) continue;
     const double c = cost(m);
     if (c < best_c) {
@@ -744,6 +900,17 @@ static b2f_status add_bluestein_pass(Builder& b, int axis, uint64_t N, const Lin
   ps.dst = dst;
   ps.label = "bluestein-fused-workgroup-stage";
   ps.route = "bluestein";
+  bool col = false;
+  if (b.fits_ip(M) && ip_layout(io, &col) &&
+      ip_begin(b, ps, IP_BLUE, col, M, N, io, flags, scale) && ip_shape(b, ps, io.inner_n, outer_n * io.mid_n, 0)) {
+    ip_grid(ps, outer_n);
+    b.set_table(b.next_pass(), Builder::F_IP_BHAT,
+                b.add_table(b.pack_complex(ip_spectrum(ps.ip.sc, chirp_spectrum(N, M)))));
+    b.set_table(b.next_pass(), Builder::F_IP_CHIRP, b.add_table(b.pack_complex(chirp_table(N))));
+    b.plan.passes.push_back(ps);
+    return B2F_OK;
+  }
+  ps.kind = Pass::BLUESTEIN;
   BluesteinParams& bp = ps.blue;
   LinesParams& lp = bp.L;
   lp.N = (uint32_t)N;
@@ -971,7 +1138,7 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
     // Rader needs p - 1 smooth and the line in one CTA; otherwise Bluestein
     // (src/runtime/rader_axis.rs:1260-1268 prefers Bluestein's register
     // kernel for non-smooth p - 1 the same way).
-    if (is_smooth13(N - 1) && b.fits_one_cta(N)) {
+    if (is_smooth13(N - 1) && b.fits_rader(N)) {
       b2f_status st = add_rader_pass(b, axis, N, io, outer_n, flags, scale, src, out_buf);
       if (st == B2F_OK) {
         *cur = out_buf;
@@ -989,7 +1156,7 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
   if (kind == AxisKind::Bluestein) {
     const uint64_t M = bluestein_length(b, N);
     b2f_status st;
-    if (b.fits_one_cta(M))
+    if (b.fits_conv(M))
       st = add_bluestein_pass(b, axis, N, io, outer_n, flags, scale, src, out_buf);
     else
       st = add_bluestein_large(b, axis, N, s, O, flags, scale, src, out_buf);
@@ -1002,7 +1169,7 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
   // Split into two passes of about sqrt(N), each a tile of many adjacent
   // columns (rows of hundreds of bytes), once enough columns exist.
   const bool split_strided = s >= 16 && N >= 2048;
-  if (b.fits_one_cta(N) && !split_strided) {
+  if (b.fits_lines(N) && !split_strided) {
     b2f_status st = add_lines_pass(b, axis, N, io, outer_n, flags, scale, src, out_buf,
                                    p2 ? "fused-pow2-workgroup-stage" : "fused-smooth-workgroup-stage",
                                    "mixed");
@@ -1038,8 +1205,8 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
   // sqrt(M) values each, split at a power of two L >= sqrt(M) (the
   // exponent splits with a shift)
   auto store_twiddles = [&](size_t idx, uint64_t M) {
-    LinesParams& lp = b.plan.passes[idx].lines;
-    lp.tw_store_M = M;
+    Pass& ps = b.plan.passes[idx];
+    (ps.kind == Pass::IP ? ps.ip.tw_store_M : ps.lines.tw_store_M) = M;
     if (!b.plan.cfg.tuning.twiddle_table) return;
     uint64_t L = 1;
     while (L * L < M) L <<= 1;
@@ -1048,7 +1215,7 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
     for (uint64_t q = 0; q < L; ++q) tb.push_back(root_fwd(q, M));
     b.set_table(idx, Builder::F_TWS_A, b.add_table(b.pack_complex(ta)));
     b.set_table(idx, Builder::F_TWS_B, b.add_table(b.pack_complex(tb)));
-    lp.d_tws = make_fastdiv((uint32_t)L);
+    (ps.kind == Pass::IP ? ps.ip.d_tws : ps.lines.d_tws) = make_fastdiv((uint32_t)L);
   };
   {
     // pass A: columns n1 (stride N2*s), W_N^{n2 k1} on store, src -> ws
@@ -1158,6 +1325,25 @@ static b2f_status add_real_pass(Builder& b, bool r2c, uint64_t N0, uint64_t nlin
   const bool even = N0 % 2 == 0;
   const uint64_t nfft = even ? N0 / 2 : N0;
   const uint64_t nbuf = even ? (r2c ? N0 / 2 : N0 / 2 + 1) : N0;
+  ps.label = r2c ? (even ? "r2c-packed-fused-stage" : "r2c-odd-fused-stage")
+                 : (even ? "c2r-packed-fused-stage" : "c2r-odd-fused-stage");
+  // even N0 whose half is not a power of two (those have fixed-length kernels)
+  if (even && (nfft & (nfft - 1)) != 0 && b.fits_ip(nfft, r2c ? nfft : 0)) {
+    Pass pi = ps;
+    if (!ip_begin(b, pi, r2c ? IP_R2C : IP_C2R, false, nfft, nfft, LineIO{},
+                  (do_scale ? PF_SCALE : 0u) | (r2c ? 0u : PF_CONJ_OUT), scale) ||
+        !ip_shape(b, pi, nlines, 1, r2c ? nfft : 0))
+      return fail(B2F_ERR_UNSUPPORTED_LENGTH, "UnsupportedLength { len: " + std::to_string(N0) + " }");
+    pi.ip.nlines = nlines;
+    pi.ip.dn = make_fastdiv((uint32_t)(nfft / 2 + 1));  // R2C: pairs k <= N / 2
+    pi.grid = (unsigned)((nlines + pi.ip.G - 1) / pi.ip.G);
+    std::vector<cd> rt(nfft);
+    const RootProduct root(N0);
+    for (uint64_t k = 0; k < nfft; ++k) rt[k] = root(k);
+    b.set_table(b.next_pass(), Builder::F_IP_RTW, b.add_table(b.pack_complex(rt)));
+    b.plan.passes.push_back(pi);
+    return B2F_OK;
+  }
   std::vector<cd> tw;
   if (!b.make_schedule(nfft, rp.sch, ps.radices, tw) || !b.fits_one_cta(nbuf))
     return fail(B2F_ERR_UNSUPPORTED_LENGTH,
@@ -1202,8 +1388,6 @@ static b2f_status add_real_pass(Builder& b, bool r2c, uint64_t N0, uint64_t nlin
   rp.dP = make_fastdiv((uint32_t)(N0 / 2 + 1));
   b.tw_table_for(rp.flags, tw, Builder::F_REAL_TW);
   ps.grid = (unsigned)((nlines + G - 1) / G);
-  ps.label = r2c ? (even ? "r2c-packed-fused-stage" : "r2c-odd-fused-stage")
-                 : (even ? "c2r-packed-fused-stage" : "c2r-odd-fused-stage");
   b.plan.passes.push_back(ps);
   return B2F_OK;
 }
@@ -1214,6 +1398,7 @@ static bool real_fast_path(const Builder& b, uint64_t N0) {
   const bool even = N0 % 2 == 0;
   const uint64_t nfft = even ? N0 / 2 : N0;
   const uint64_t nbuf = even ? N0 / 2 + 1 : N0;
+  if (even && (nfft & (nfft - 1)) != 0 && is_smooth13(nfft) && b.fits_ip(nfft, nfft)) return true;
   return !stage_radices(nfft).empty() && b.fits_one_cta(nbuf) && N0 >= 2;
 }
 
@@ -1370,13 +1555,15 @@ static void build_diagnostics(Plan& plan) {
   os << "],\"stages\":[";
   for (size_t i = 0; i < plan.passes.size(); ++i) {
     const Pass& p = plan.passes[i];
-    const char* kind = p.kind == Pass::LINES ? "lines" : p.kind == Pass::POW2 ? (p.colmajor ? "register-pow2-columns" : "register-pow2-lines") : p.kind == Pass::RADER ? "rader"
+    const char* kind = p.kind == Pass::IP ? (p.ip_kind == IP_LINES ? "lines" : p.ip_kind == IP_RADER ? "rader"
+                            : p.ip_kind == IP_BLUE ? "bluestein" : p.ip_kind == IP_R2C ? "r2c" : "c2r")
+                     : p.kind == Pass::LINES ? "lines" : p.kind == Pass::POW2 ? (p.colmajor ? "register-pow2-columns" : "register-pow2-lines") : p.kind == Pass::RADER ? "rader"
                      : p.kind == Pass::BLUESTEIN ? "bluestein" : p.kind == Pass::R2C ? "r2c"
                      : p.kind == Pass::C2R ? "c2r" : p.kind == Pass::BLUE_ELEM ? "bluestein-elementwise"
                      : p.kind == Pass::REAL_ELEM ? "real-elementwise"
                      : p.kind == Pass::TC_DFT64 ? "tensor-core-dft"
                      : p.kind == Pass::SMALL_VOLUME ? "small-volume" : "scale-copy";
-    uint32_t G = (p.kind == Pass::LINES || p.kind == Pass::POW2) ? p.lines.G : p.kind == Pass::RADER ? p.rader.L.G
+    uint32_t G = p.kind == Pass::IP ? p.ip.G : (p.kind == Pass::LINES || p.kind == Pass::POW2) ? p.lines.G : p.kind == Pass::RADER ? p.rader.L.G
                : p.kind == Pass::BLUESTEIN ? p.blue.L.G : (p.kind == Pass::R2C || p.kind == Pass::C2R) ? p.real.G : 0;
     os << (i ? "," : "") << "{\"label\":\"" << json_escape(p.label) << "\",\"kind\":\"" << kind
        << "\",\"route\":\"" << p.route << "\",\"axis\":" << p.axis << ",\"radices\":[";
@@ -1385,6 +1572,8 @@ static void build_diagnostics(Plan& plan) {
        << ",\"smem_bytes\":" << p.smem << ",\"src\":" << p.src << ",\"dst\":" << p.dst;
     if (p.kind == Pass::BLUESTEIN) os << ",\"convolution_length\":" << p.blue.M;
     if (p.kind == Pass::RADER) os << ",\"convolution_length\":" << (p.rader.L.N - 1);
+    if (p.kind == Pass::IP && (p.ip_kind == IP_RADER || p.ip_kind == IP_BLUE))
+      os << ",\"convolution_length\":" << p.ip.sc.N;
     if (p.tma) os << ",\"tma_tiles\":true,\"persistent_grid\":" << p.tma_grid;
     os << "}";
   }
@@ -1665,6 +1854,11 @@ static b2f_status run_passes(const Plan& plan, cudaStream_t st, const void* in, 
           e = launch_r2c(plan.prec, p.real, p.grid, p.threads, p.smem, st);
         else
           e = launch_c2r(plan.prec, p.real, p.grid, p.threads, p.smem, st);
+        break;
+      case Pass::IP:
+        p.ip.in = src;
+        p.ip.out = dst;
+        e = launch_ip(plan.prec, p.ip_kind, p.ip_col, p.ip, p.grid, p.threads, p.smem, st);
         break;
       case Pass::SCALE_COPY:
         e = launch_scale_copy(plan.prec, src, dst, p.copy_n, p.copy_scale, p.copy_conj, st);

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/wgpufft_b200.h"
+#include "ipfft.h"
 #include "kernels.h"
 
 namespace b2f {
@@ -64,7 +65,7 @@ constexpr int kNumWorkspaces = 6;
 
 struct Pass {
   enum Kind { LINES, POW2, RADER, BLUESTEIN, R2C, C2R, SCALE_COPY, BLUE_ELEM, REAL_ELEM, TC_DFT64,
-              SMALL_VOLUME } kind = LINES;
+              SMALL_VOLUME, IP } kind = LINES;
   int pow2_E = 16;         // POW2: values per thread
   bool colmajor = false;   // POW2: adjacent lines first
   std::string label;  // stage label (diagnostics)
@@ -81,6 +82,9 @@ struct Pass {
   BlueElemParams belem{};
   RealElemParams relem{};
   SmallVolumeParams svol{};
+  IpParams ip{};          // IP: the in-place mixed-radix kernels
+  IpKind ip_kind = IP_LINES;
+  bool ip_col = false;
   uint64_t copy_n = 0;
   double copy_scale = 1.0;
   bool copy_conj = false;
