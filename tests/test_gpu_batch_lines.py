@@ -1,0 +1,50 @@
+"""The batch kernels at the edges of their ranges: lines of one CTA (tiny,
+smooth, Rader, Bluestein) up to the longest that fits, the shortest
+and longest lines of the two- and three-pass routes, one ragged column or
+row, passes of two to four stages, prime powers, and Bluestein lines whose
+convolution is odd, against numpy in 64 bits (bound of every f32 route:
+2e-6 in the 2-norm)."""
+import numpy as np
+import pytest
+import torch
+
+import wgpufft_b200 as w
+from wgpufft_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [1, 2, 13, 16, 17, 18, 19, 23, 34, 94, 97, 337, 1000, 1409, 2521, 2731, 2777, 2801, 5600, 5616, 2816, 3024, 4394, 6561, 6655, 14641, 15625, 16807, 28561, 65536, 131072, 262144, 250000,
+           200200, 1409, 1418, 2837, 2999, 8200, 34607, 65521, 65537, 99990, 116033]
+
+
+@pytest.mark.parametrize("inverse", [False, True])
+@pytest.mark.parametrize("repeat", [1, 3])
+def test_long_lines(inverse, repeat):
+    lengths = np.array(LENGTHS * repeat)
+    off = workloads.packed_offsets(lengths)
+    x = workloads.normal_complex(int(lengths.sum()), 17)
+    d = torch.from_numpy(x).cuda()
+    out = torch.empty_like(d)
+    b = w.FftBatch(lengths, off, direction=w.FftDirection.Inverse if inverse else w.FftDirection.Forward)
+    b.execute(d, out)
+    y = out.cpu().numpy()
+    for n, o in zip(lengths, off):
+        z = x[o:o + n].astype(np.complex128)
+        ref = np.fft.ifft(z) if inverse else np.fft.fft(z)
+        assert np.linalg.norm(y[o:o + n] - ref) <= 2e-6 * np.linalg.norm(ref), n
+    b.execute(d, d)  # in place
+    assert torch.equal(d, out)
+
+
+def test_a_line_alone_equals_the_same_line_among_others():
+    n = 30011
+    x = torch.from_numpy(workloads.normal_complex(n, 3)).cuda()
+    alone = torch.empty_like(x)
+    w.FftBatch([n], [0]).execute(x, alone)
+    lengths = np.array([20000, n, 65521, 4096])
+    off = workloads.packed_offsets(lengths)
+    d = torch.zeros(int(lengths.sum()), dtype=torch.complex64, device="cuda")
+    d[off[1]:off[1] + n] = x
+    out = torch.empty_like(d)
+    w.FftBatch(lengths, off).execute(d, out)
+    assert torch.equal(out[off[1]:off[1] + n], alone)

@@ -26,6 +26,15 @@ static bool smooth7(uint64_t n) {
   return n == 1;
 }
 
+static std::vector<float> pack_f32(const std::vector<cd>& v) {
+  std::vector<float> f(v.size() * 2);
+  for (size_t i = 0; i < v.size(); ++i) {
+    f[2 * i] = (float)v[i].real();
+    f[2 * i + 1] = (float)v[i].imag();
+  }
+  return f;
+}
+
 static uint32_t ld_f32(uint64_t n) { return (uint32_t)(n + (n >> 4) + 1); }
 
 static Schedule schedule_for(uint64_t n) {
@@ -135,7 +144,7 @@ struct BatchPlan {
   cudaStream_t hs[3] = {nullptr, nullptr, nullptr};  // copy in, transform, copy out
   cudaEvent_t hev_start = nullptr, hev_done = nullptr;
   cudaEvent_t hev_in[kHostChunks] = {}, hev_c[kHostChunks] = {};
-  uint32_t long_cap = 0;
+  uint32_t long_cap = 0, long_tab = 0;  // values of data and of tables a task needs
   size_t smem_long = 0;
   unsigned grid_long = 0;
   uint64_t lines_long = 0, elems_long = 0;
@@ -192,76 +201,77 @@ constexpr unsigned kClusterThreads = 512;
 struct LenInfo {
   BatchLen d;
   std::vector<cd> bhat;
-  std::vector<uint32_t> pin, pout;
+  std::vector<uint32_t> perm;  // Rader: g^q
+  std::vector<cd> chirp;       // CTA Bluestein
   double cost = 0;
   LongLenDesc lng;      // long kinds
-  Schedule s1, s2;      // long kinds: schedules of N1 and N2
 };
 
 
-// Lines per task of a long-line pass of length nx (log2): 16 up to 208
-// points, 8 up to 393, 4 up to 512, so that a task's buffer of nx*(G+1)
-// values stays within 3540 (three buffers and the two table areas of two
-// CTAs fit one SM).
-static uint32_t long_lines_log2(uint64_t nx) { return nx <= 208 ? 4 : (nx <= 393 ? 3 : 2); }
-
-// Estimated cost of one task of a long-line pass of length nx (2..512,
-// 13-smooth): for each stage of radix R, the butterfly rounds the task's 256
-// threads take (ceil(NR / S) rounds of S threads per line, idle threads
-// included) times R points each, weighted by an instruction estimate per
-// point (about 10 for the shared-memory traffic, addressing and twiddle
-// product, plus the radix-R codelet's arithmetic).  0 for other lengths.
-static const std::vector<double>& long_task_costs() {
-  static const std::vector<double> tab = [] {
-    std::vector<double> t(513, 0.0);
-    for (uint32_t nx = 2; nx <= 512; ++nx) {
-      const std::vector<uint32_t> rad = stage_radices(nx);
-      if (rad.empty()) continue;
-      const uint32_t S = kLongThreads >> long_lines_log2(nx);
-      double c = 0;
-      for (uint32_t R : rad) {
-        double f = 0;
-        switch (R) {
-          case 2: f = 2.0; break;
-          case 3: case 4: f = 4.0; break;
-          case 5: f = 6.4; break;
-          case 7: f = 10.3; break;
-          case 8: f = 6.5; break;
-          case 9: f = 8.9; break;
-          case 11: f = 12.7; break;
-          case 13: f = 13.8; break;
-          default: f = 9.0; break;  // 16
-        }
-        const uint32_t rounds = (nx / R + S - 1) / S;
-        c += (double)rounds * R * kLongThreads * (10.0 + f);
-      }
-      t[nx] = c;
-    }
+// Radices of a long-line pass of nx points (two stages at least), by nx;
+// empty where there are none.
+static const std::vector<std::vector<uint32_t>>& long_radices() {
+  static const std::vector<std::vector<uint32_t>> tab = [] {
+    std::vector<std::vector<uint32_t>> t(513);
+    for (uint32_t nx = 4; nx <= 512; ++nx) t[nx] = ip_radices(nx, 2);
     return t;
   }();
   return tab;
 }
 
-// Estimated cost of a long line over T = a * (T / a): `ffts` transforms
-// through both passes (1 for a smooth line; 2 for Bluestein, forward and
-// inverse) and `passes` HBM passes of about 30 instructions per point.
-static double long_cost(uint64_t T, uint64_t a, int ffts, int passes) {
-  const std::vector<double>& t = long_task_costs();
-  const uint64_t b = T / a;
-  const uint64_t Ga = 1u << long_lines_log2(a), Gb = 1u << long_lines_log2(b);
-  return ffts * (t[a] * (double)((b + Ga - 1) / Ga) + t[b] * (double)((a + Gb - 1) / Gb)) +
-         passes * 30.0 * (double)T;
+// Columns or rows of nx points a task takes when a line has `across` of
+// them: the power of two that fills `values` (a row's sub-lines have an odd
+// pitch), no wider than the line needs.  (Fuller tasks keep the 256 threads
+// busy: a task of 16 columns of 50 points has 50 radix-16 butterflies for
+// them.)
+static uint32_t long_lines(uint64_t nx, uint64_t across, bool row,
+                           uint64_t values = kLongTaskValues) {
+  uint64_t line = nx;
+  if (row) {
+    const std::vector<uint32_t>& r = long_radices()[nx];
+    const uint64_t R0 = *std::max_element(r.begin(), r.end());
+    line = (R0 * ip_pitch((uint32_t)(nx / R0))) | 1u;
+  }
+  uint32_t G = 4;
+  while (2 * G * line <= values && G < across && G < 256) G *= 2;
+  return G;
 }
 
-// T = N1 * N2 with both factors 13-smooth in [2, 512]: the split of the
-// lowest estimated cost (*cost); 0 when none exists.
-static uint64_t long_split(uint64_t T, int ffts = 1, int passes = 2, double* cost = nullptr) {
-  const std::vector<double>& t = long_task_costs();
+// Estimated cost of the pass of nx points over `across` columns or rows:
+// for each stage of radix R the butterfly rounds of the 256 threads (idle
+// ones included) times R points at ip_cost's instruction estimate, and
+// about 30 instructions a value held for the loads, stores and twiddles.
+static double long_pass_cost(uint64_t nx, uint64_t across, int ffts, bool row) {
+  static const std::vector<double> stage = [] {
+    std::vector<double> t(17, 0.0);
+    for (uint32_t R = 2; R <= 16; ++R) t[R] = ip_cost({R});
+    return t;
+  }();
+  const uint64_t G = long_lines(nx, across, row);
+  const double tasks = (double)((across + G - 1) / G);
+  double c = 0;
+  for (uint32_t R : long_radices()[nx])
+    c += (double)((G * nx / R + kLongThreads - 1) / kLongThreads) * kLongThreads * R * stage[R];
+  return tasks * (ffts * c + 30.0 * (double)(G * nx));
+}
+
+// Estimated cost of a long line over T = a * (T / a): `ffts` transforms
+// through both passes (1 for a smooth line; 2 for Bluestein: the column
+// pass twice, the row pass once with both).
+static double long_cost(uint64_t T, uint64_t a, int ffts) {
+  const uint64_t b = T / a;
+  return ffts * long_pass_cost(a, b, 1, false) + long_pass_cost(b, a, ffts, true);
+}
+
+// T = N1 * N2 with both factors 13-smooth, composite and up to 512: the
+// split of the lowest estimated cost (*cost); 0 when none exists.
+static uint64_t long_split(uint64_t T, int ffts = 1, double* cost = nullptr) {
+  const auto& rad = long_radices();
   uint64_t best_a = 0;
   double best = 1e300;
-  for (uint64_t a = 2; a <= 512; ++a) {
-    if (T % a || T / a > 512 || T / a < 2 || t[a] == 0 || t[T / a] == 0) continue;
-    const double c = long_cost(T, a, ffts, passes);
+  for (uint64_t a = 4; a <= 512; ++a) {
+    if (T % a || T / a > 512 || T / a < 4 || rad[a].empty() || rad[T / a].empty()) continue;
+    const double c = long_cost(T, a, ffts);
     if (c < best) {
       best = c;
       best_a = a;
@@ -271,8 +281,44 @@ static uint64_t long_split(uint64_t T, int ffts = 1, int passes = 2, double* cos
   return best_a;
 }
 
-// Long-line descriptor of length N over the transform length T = n1 * (T / n1)
-// (pass lengths <= 512, so at most 9 stages each).
+// Appends the in-place stage twiddles of length n to tw (at an even index)
+// once per (length, layout), and describes the passes of G lines over it.
+using LongCache = std::map<std::pair<uint32_t, bool>, std::pair<IpSched, uint64_t>>;
+static void long_pass_tables(IpRows& q, uint32_t n, bool row, uint32_t G, bool lines_first,
+                             std::vector<cd>& tw, uint64_t base, LongCache& cache) {
+  auto it = cache.find({n, row});
+  if (it == cache.end()) {
+    if ((base + tw.size()) % 2) tw.push_back(cd(0.0, 0.0));
+    const uint64_t at = base + tw.size();
+    std::vector<uint32_t> rad;
+    std::vector<cd> t;
+    IpSched sc;
+    ip_schedule(n, row, true, 2, sc, rad, t);
+    tw.insert(tw.end(), t.begin(), t.end());
+    it = cache.emplace(std::make_pair(n, row), std::make_pair(sc, at)).first;
+  }
+  q.sc = it->second.first;
+  q.sc.tw0 += (uint32_t)it->second.second;
+  for (uint32_t s = 0; s < q.sc.nst; ++s) q.sc.st[s].tw += (uint32_t)it->second.second;
+  q.flags = lines_first ? (uint32_t)PF_CFIRST_STORE : 0u;
+  q.G = G;
+  q.lam = G * q.sc.R0;
+  q.dlam = make_fastdiv(q.lam);
+  q.dG = make_fastdiv(G);
+  q.pitch = ip_pitch(q.sc.NS);
+  // rows stored lines first read across the lines: an odd line pitch
+  q.LDl = row ? q.sc.R0 * q.pitch | (lines_first ? 1u : 0u) : 0u;
+}
+
+// Columns and rows a task of the line, tasks of at most `values` values.
+static void set_long_tasks(LongLenDesc& g, uint64_t values) {
+  g.c.G = long_lines(g.N1, g.N2, false, values);
+  g.r.G = long_lines(g.N2, g.N1, true, values);
+}
+
+// Long-line descriptor of length N over the transform length T = n1 * (T /
+// n1).  The radices of both passes are known by their lengths, so a
+// Bluestein line's spectrum can be put in its rows' order here.
 static void set_long(LenInfo& li, uint64_t N, uint64_t T, uint64_t n1, bool blue) {
   BatchLen& d = li.d;
   LongLenDesc& g = li.lng;
@@ -284,12 +330,42 @@ static void set_long(LenInfo& li, uint64_t N, uint64_t T, uint64_t n1, bool blue
   g.M = (uint32_t)T;
   g.N1 = (uint32_t)n1;
   g.N2 = (uint32_t)(T / n1);
-  g.lgc = long_lines_log2(g.N1);
-  g.lgr = long_lines_log2(g.N2);
+  set_long_tasks(g, kLongTaskValues);
   g.blue = blue ? 1u : 0u;
   g.scale = d.scale;
-  li.s1 = schedule_for(g.N1);
-  li.s2 = schedule_for(g.N2);
+  // n^2 mod 2N (mod_square)
+  uint32_t b = 0;
+  while ((2ull << b) <= 2 * N) ++b;
+  g.minv = (uint32_t)(((1ull << (32 + b)) - 1) / (2 * N));
+  g.mshift = b - 2;
+}
+
+// A convolution's spectrum in the order its frequencies take in a row of n
+// points ([pos][k0]).
+static std::vector<cd> row_spectrum(uint64_t n, const std::vector<cd>& bhat) {
+  IpSched sc;
+  std::vector<uint32_t> rad;
+  std::vector<cd> unused, out(bhat.size());
+  ip_schedule(n, true, true, 2, sc, rad, unused);
+  for (uint32_t pos = 0; pos < sc.NS; ++pos)
+    for (uint32_t k0 = 0; k0 < sc.R0; ++k0)
+      out[(size_t)pos * sc.R0 + k0] = bhat[ip_frequency(sc, k0, pos)];
+  return out;
+}
+
+// The spectrum of a long Bluestein line, row k1 at k1 * N2 in the order the
+// row's frequencies take: entry [pos][k0] holds bin k1 + N1 * k2.
+static std::vector<cd> long_spectrum(const LongLenDesc& g, const std::vector<cd>& bhat) {
+  IpSched sc;
+  std::vector<uint32_t> rad;
+  std::vector<cd> unused, out(bhat.size());
+  ip_schedule(g.N2, true, true, 2, sc, rad, unused);
+  std::vector<uint32_t> k2(g.N2);
+  for (uint32_t pos = 0; pos < sc.NS; ++pos)
+    for (uint32_t k0 = 0; k0 < sc.R0; ++k0) k2[pos * sc.R0 + k0] = ip_frequency(sc, k0, pos);
+  for (uint64_t k1 = 0; k1 < g.N1; ++k1)
+    for (uint64_t i = 0; i < g.N2; ++i) out[k1 * g.N2 + i] = bhat[k1 + (uint64_t)g.N1 * k2[i]];
+  return out;
 }
 
 // The two-level tables of a long line (appended to tw; offsets relative to
@@ -298,18 +374,49 @@ static void set_long(LenInfo& li, uint64_t N, uint64_t T, uint64_t n1, bool blue
 // Bluestein lines the chirp W_2N likewise, so the kernel splits an exponent
 // with a shift and a mask (M <= 512 * 512 keeps both within 512 values).
 static void long_split_tables(LongLenDesc& g, std::vector<cd>& tw, uint64_t base) {
-  auto two_level = [&](uint64_t M, uint32_t* ta, uint32_t* tb, uint32_t* split) {
+  auto two_level = [&](uint64_t M, uint32_t* ta, uint32_t* tb, uint32_t* tn, uint32_t* split) {
     uint32_t sh = 0;
     while ((1ull << (2 * sh)) < M) ++sh;
     const uint64_t L = 1ull << sh;
     *split = sh;
     *ta = (uint32_t)(base + tw.size());
+    *tn = (uint32_t)((M + L - 1) / L);
     for (uint64_t a = 0; a * L < M; ++a) tw.push_back(root_fwd(a * L, M));
     *tb = (uint32_t)(base + tw.size());
     for (uint64_t b = 0; b < L; ++b) tw.push_back(root_fwd(b, M));
   };
-  two_level(g.M, &g.ta, &g.tb, &g.tsplit);
-  if (g.blue) two_level(2ull * g.N, &g.ca, &g.cb, &g.csplit);
+  two_level(g.M, &g.ta, &g.tb, &g.tn, &g.tsplit);
+  if (g.blue) two_level(2ull * g.N, &g.ca, &g.cb, &g.cn, &g.csplit);
+}
+
+// Stage tables of both passes and the two-level tables of a long line.
+static void long_tables_of(LongLenDesc& g, std::vector<cd>& tw, uint64_t base, LongCache& cache) {
+  long_pass_tables(g.c, g.N1, false, g.c.G, false, tw, base, cache);
+  long_pass_tables(g.r, g.N2, true, g.r.G, !g.blue, tw, base, cache);
+  long_split_tables(g, tw, base);
+}
+
+// Shared memory of a long line's task in phase ph (1..3): its data, its
+// two-level tables.
+static uint32_t long_task_values(const LongLenDesc& g, int ph) {
+  return ph == 2 ? g.r.G * g.r.LDl : g.c.G * g.N1;
+}
+static uint32_t long_table_values(const LongLenDesc& g, int ph) {
+  uint32_t n = 0;
+  if (ph != 3) n += g.tn + (1u << g.tsplit);
+  if (g.blue && ph != 2) n += g.cn + (1u << g.csplit);
+  return n;
+}
+
+// The stage tables of a CTA length and its in-place description.
+static void cta_tables_of(BatchLen& d, std::vector<cd>& tw, uint64_t base, LongCache& cache) {
+  long_pass_tables(d.ip, d.M, true, d.G, false, tw, base, cache);
+}
+
+// Values of shared memory a CTA task takes.
+static uint32_t cta_task_values(const BatchLen& d) {
+  if (d.ip.sc.N == 0) return 2 * d.G * d.LD;
+  return d.G * (d.ip.LDl + (d.kind == BK_RADER ? d.N + 2 : 0));
 }
 
 // Chooses the execution of one distinct length.
@@ -326,13 +433,19 @@ static bool classify(uint64_t N, int32_t direction, int32_t normalization, size_
     sc = 1.0f / sqrtf((float)N);
   d.scale = sc;
   d.dN = make_fastdiv((uint32_t)N);
-  const auto cta_bytes = [](uint64_t lbuf) { return 2 * (size_t)ld_f32(lbuf) * 8; };
+  // bytes of a line in a CTA task (in place; up to 16 points two ping-pong
+  // buffers), with `extra` values beside the transform's buffer, and of a
+  // cluster rank's two buffers
+  const auto cta_bytes = [](uint64_t n, uint64_t extra = 0) {
+    return n <= 16 ? 2 * (size_t)ld_f32(n) * 8 : (size_t)(n + 17 + extra) * 8;
+  };
+  const auto cl_bytes = [](uint64_t lbuf) { return 2 * (size_t)ld_f32(lbuf) * 8; };
   uint64_t n1 = 0;
   if (is_smooth13(N) && cta_bytes(N) > cta_cap && !clusters) n1 = long_split(N);
   uint32_t cl_split = 0;
   if (clusters && is_smooth13(N) && cta_bytes(N) > cta_cap)
     for (uint32_t P : {8u, 7u, 5u, 4u, 3u, 2u})
-      if (N % P == 0 && cta_bytes(N / P) <= cl_cap) {
+      if (N % P == 0 && cl_bytes(N / P) <= cl_cap) {
         cl_split = P;
         break;
       }
@@ -351,36 +464,46 @@ static bool classify(uint64_t N, int32_t direction, int32_t normalization, size_
   if (smooth && cta_bytes(N) <= cta_cap) {
     d.kind = BK_MIXED;
     d.M = (uint32_t)N;
-    d.LD = ld_f32(N);
-    d.sch = schedule_for(N);
+    if (N <= 16) {
+      d.LD = ld_f32(N);
+      d.sch = schedule_for(N);
+    }
   } else if (smooth) {
     set_long(li, N, N, n1, false);
-  } else if (is_prime_u64(N) && N >= 3 && is_smooth13(N - 1) && cta_bytes(N) <= cta_cap) {
+  } else if (is_prime_u64(N) && N >= 17 && is_smooth13(N - 1) && cta_bytes(N - 1, N + 2) <= cta_cap) {
     d.kind = BK_RADER;
     d.M = (uint32_t)(N - 1);
-    d.LD = ld_f32(N);
-    d.sch = schedule_for(N - 1);
-    d.dP1 = make_fastdiv((uint32_t)(N - 1));
     const uint64_t g = primitive_root(N), ginv = mod_pow64(g, N - 2, N);
-    li.pin.resize(N - 1);
-    li.pout.resize(N - 1);
+    li.perm.resize(N - 1);
     li.bhat.resize(N - 1);
     uint64_t v = 1;
     for (uint64_t q = 0; q + 1 < N; ++q) {
-      li.pin[q] = (uint32_t)v;
+      li.perm[q] = (uint32_t)v;
       v = v * g % N;
     }
     v = 1;
     for (uint64_t r = 0; r + 1 < N; ++r) {
-      li.pout[v - 1] = (uint32_t)r;
       li.bhat[r] = root_fwd(v, N);
       v = v * ginv % N;
     }
     host_fft_fwd(li.bhat);
     for (auto& x : li.bhat) x /= (double)(N - 1);
+    li.bhat = row_spectrum(N - 1, li.bhat);
   } else {
     uint64_t M = 2 * N - 1;
     while (!smooth7(M)) ++M;
+    if (cta_bytes(M) <= cta_cap) {
+      // up to 2.25 N, the 7-smooth length of the cheapest stages that fits
+      double best = 1e300;
+      for (uint64_t m = M, end = 9 * N / 4; m <= std::max(M, end) && cta_bytes(m) <= cta_cap; ++m) {
+        if (!smooth7(m)) continue;
+        const double c = ip_cost(ip_radices(m, 2)) * (double)m;
+        if (c < best) {
+          best = c;
+          M = m;
+        }
+      }
+    }
     uint64_t mlong = 0, a = 0;
     if (cta_bytes(M) > cta_cap && !clusters) {
       // the 13-smooth convolution length in [2N - 1, 2.25 N] (and its split
@@ -390,7 +513,7 @@ static bool classify(uint64_t N, int32_t direction, int32_t normalization, size_
       for (uint64_t m = 2 * N - 1; m <= 262144 && (m <= 9 * N / 4 || !mlong); ++m) {
         if (!is_smooth13(m)) continue;
         double c = 0;
-        const uint64_t am = long_split(m, 2, 3, &c);
+        const uint64_t am = long_split(m, 2, &c);
         if (am && c < best) {
           best = c;
           mlong = m;
@@ -401,8 +524,6 @@ static bool classify(uint64_t N, int32_t direction, int32_t normalization, size_
     if (cta_bytes(M) <= cta_cap) {
       d.kind = BK_BLUE;
       d.M = (uint32_t)M;
-      d.LD = ld_f32(M);
-      d.sch = schedule_for(M);
     } else if (mlong) {
       M = mlong;
       set_long(li, N, M, a, true);
@@ -411,11 +532,11 @@ static bool classify(uint64_t N, int32_t direction, int32_t normalization, size_
       uint32_t P = kClusterP;
       uint64_t L = (2 * N - 1 + P - 1) / P;
       while (!smooth7(L)) ++L;
-      if (cta_bytes(L) > cl_cap) {
+      if (cl_bytes(L) > cl_cap) {
         P = kClusterBig;
         L = (2 * N - 1 + P - 1) / P;
         while (!smooth7(L)) ++L;
-        if (cta_bytes(L) > cl_cap) return false;
+        if (cl_bytes(L) > cl_cap) return false;
       }
       M = L * P;
       d.kind = BK_CL_BLUE;
@@ -425,18 +546,23 @@ static bool classify(uint64_t N, int32_t direction, int32_t normalization, size_
       d.LD = ld_f32(L);
       d.sch = schedule_for(L);
     }
-    d.dM = make_fastdiv((uint32_t)M);
-    d.dMN = make_fastdiv((uint32_t)(M - N));
     li.bhat = chirp_spectrum(N, M);
+    if (d.kind == BK_LONG_BLUE) li.bhat = long_spectrum(li.lng, li.bhat);
+    if (d.kind == BK_BLUE) {
+      li.bhat = row_spectrum(M, li.bhat);
+      const RootProduct root(2 * N);
+      li.chirp.resize(N);
+      for (uint64_t n = 0; n < N; ++n) li.chirp[n] = root(n * n % (2 * N));
+    }
   }
   const double T = d.M;
   li.cost = T * std::log2(std::max(2.0, T)) * (d.kind == BK_BLUE || d.kind == BK_CL_BLUE ? 3 : 1);
   if (d.kind == BK_LONG || d.kind == BK_LONG_BLUE) {
     d.G = 1;
   } else if (d.kind == BK_MIXED || d.kind == BK_RADER || d.kind == BK_BLUE) {
-    uint64_t G = std::max<uint64_t>(1, 4096 / d.M);
-    G = std::min<uint64_t>(G, kBatchMaxG);
-    while (G > 1 && G * cta_bytes(d.kind == BK_RADER ? N : d.M) > cta_cap) --G;
+    // lines that fill the CTA's share
+    const size_t line = d.kind == BK_RADER ? cta_bytes(N - 1, N + 2) : cta_bytes(d.M);
+    const uint64_t G = std::max<uint64_t>(1, std::min<uint64_t>(cta_cap / line, kBatchMaxG));
     d.G = (uint32_t)G;
   } else {
     d.G = 1;
@@ -531,24 +657,34 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
                   "UnsupportedLength { len: " + std::to_string(lens_list[i]) + " } in a batch");
     }
   bp->distinct = lens_list.size();
+  // A batch with few long lines takes smaller tasks, so that a phase has
+  // three tasks for each of the CTAs that fit (four an SM): 100 lines of
+  // 1,400 to 2,300 points as one task a line and phase took 132 us against
+  // 91 with several.  (The values a task holds do not change a line's
+  // arithmetic.)
+  for (uint64_t values = kLongTaskValues; values >= 512; values /= 2) {
+    uint64_t tasks = 0;
+    for (size_t i = 0; i < infos.size(); ++i) {
+      if (infos[i].d.kind != BK_LONG && infos[i].d.kind != BK_LONG_BLUE) continue;
+      LongLenDesc& g = infos[i].lng;
+      set_long_tasks(g, values);
+      tasks += by_len[lens_list[i]].size() * ((g.N2 + g.c.G - 1) / g.c.G);
+    }
+    if (tasks >= 3 * 4 * 148) break;
+  }
   // twiddle tables shared by every length of the batch
   {
     std::vector<cd> tw;
     std::map<uint32_t, uint32_t> cache;
+    LongCache long_cache;
     for (auto& li : infos) {
       BatchLen& d = li.d;
       if (d.kind == BK_LONG || d.kind == BK_LONG_BLUE) {
-        // stage tables of both passes and W_M^{a N2} / W_M^b
-        LongLenDesc& g = li.lng;
-        attach_stage_table(li.s1, tw, cache);
-        attach_stage_table(li.s2, tw, cache);
-        for (int w = 0; w < 2; ++w) {
-          const Schedule& sc = w ? li.s2 : li.s1;
-          LongSched& ls = w ? g.s2 : g.s1;
-          ls.nst = sc.nst;
-          for (uint32_t k = 0; k < sc.nst; ++k) ls.st[k] = sc.st[k];
-        }
-        long_split_tables(g, tw, 0);
+        long_tables_of(li.lng, tw, 0, long_cache);
+        continue;
+      }
+      if (d.kind != BK_CL_MIXED && d.kind != BK_CL_BLUE && (d.kind != BK_MIXED || d.N > 16)) {
+        cta_tables_of(d, tw, 0, long_cache);
         continue;
       }
       attach_stage_table(d.sch, tw, cache);
@@ -595,12 +731,18 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
       li.d.bhat = (const c32*)p;
       li.lng.bhat = (const c32*)p;
     }
-    if (!li.pin.empty()) {
-      void *a, *b;
-      if (!upload(li.pin.data(), li.pin.size() * 4, &a) || !upload(li.pout.data(), li.pout.size() * 4, &b))
+    if (!li.perm.empty()) {
+      void* a;
+      if (!upload(li.perm.data(), li.perm.size() * 4, &a))
         return fail(B2F_ERR_RESOURCE_ALLOCATION, "batch table allocation failed");
-      li.d.perm_in = (const uint32_t*)a;
-      li.d.perm_out = (const uint32_t*)b;
+      li.d.perm = (const uint32_t*)a;
+    }
+    if (!li.chirp.empty()) {
+      const std::vector<float> f = pack_f32(li.chirp);
+      void* a;
+      if (!upload(f.data(), f.size() * 4, &a))
+        return fail(B2F_ERR_RESOURCE_ALLOCATION, "batch table allocation failed");
+      li.d.chirp = (const c32*)a;
     }
   }
   // chunks of host execution: lines in offset order, cut into runs of about
@@ -693,7 +835,7 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
     const bool cl = d.kind == BK_CL_MIXED || d.kind == BK_CL_BLUE;
     if (d.kind == BK_LONG || d.kind == BK_LONG_BLUE) {
       const LongLenDesc& g = infos[li].lng;
-      const uint32_t Gc = 1u << g.lgc, Gr = 1u << g.lgr;
+      const uint32_t Gc = g.c.G, Gr = g.r.G;
       for (uint64_t line : lines) {
         const uint64_t lbase = offsets[line], lscr = scratch_total;
         ++n_long_lines;
@@ -833,15 +975,17 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
     if (d.kind == BK_CL_MIXED || d.kind == BK_CL_BLUE) buf_cl = std::max(buf_cl, d.LD);
     else if (d.kind == BK_LONG || d.kind == BK_LONG_BLUE) {
       const LongLenDesc& g = li.lng;
-      bp->long_cap = std::max(bp->long_cap, g.N1 * ((1u << g.lgc) + 1));
-      bp->long_cap = std::max(bp->long_cap, g.N2 * ((1u << g.lgr) + 1));
+      for (int ph = 1; ph <= 3; ++ph) {
+        bp->long_cap = std::max(bp->long_cap, long_task_values(g, ph));
+        bp->long_tab = std::max(bp->long_tab, long_table_values(g, ph));
+      }
     } else {
-      buf_cta = std::max<uint32_t>(buf_cta, d.G * d.LD);
+      buf_cta = std::max<uint32_t>(buf_cta, cta_task_values(d));
     }
   }
   bp->buf_cta = buf_cta;
   bp->buf_cl = buf_cl;
-  bp->smem_cta = 2 * (size_t)buf_cta * 8 + 2 * kBatchMaxG * 8;
+  bp->smem_cta = (size_t)buf_cta * 8;
   bp->smem_cl = 2 * (size_t)buf_cl * 8;
   // device arrays
   std::vector<BatchLen> dl(infos.size());
@@ -898,7 +1042,7 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
     bp->grid_cta = (unsigned)std::min<uint64_t>((uint64_t)nsm * per_sm, bp->n_cta);
   }
   if (n_long_lines) {
-    bp->smem_long = (3 * (size_t)bp->long_cap + 2 * kLongTab) * 8;
+    bp->smem_long = ((size_t)bp->long_cap + bp->long_tab) * 8;
     if (set_smem(k_long_pass<1>, bp->smem_long) != cudaSuccess ||
         set_smem(k_long_pass<2>, bp->smem_long) != cudaSuccess ||
         set_smem(k_long_pass<3>, bp->smem_long) != cudaSuccess)
@@ -1233,19 +1377,13 @@ static void length_twiddles(LenInfo& li, std::vector<cd>& tw, uint64_t base) {
   std::map<uint32_t, uint32_t> cache;
   BatchLen& d = li.d;
   if (d.kind == BK_LONG || d.kind == BK_LONG_BLUE) {
-    LongLenDesc& g = li.lng;
-    attach_stage_table(li.s1, tw, cache);
-    attach_stage_table(li.s2, tw, cache);
-    for (int w = 0; w < 2; ++w) {
-      const Schedule& sc = w ? li.s2 : li.s1;
-      LongSched& ls = w ? g.s2 : g.s1;
-      ls.nst = sc.nst;
-      for (uint32_t k = 0; k < sc.nst; ++k) {
-        ls.st[k] = sc.st[k];
-        ls.st[k].tw_off += (uint32_t)base;
-      }
-    }
-    long_split_tables(g, tw, base);
+    LongCache long_cache;
+    long_tables_of(li.lng, tw, base, long_cache);
+    return;
+  }
+  if (d.kind != BK_MIXED || d.N > 16) {
+    LongCache long_cache;
+    cta_tables_of(d, tw, base, long_cache);
     return;
   }
   attach_stage_table(d.sch, tw, cache);
@@ -1290,9 +1428,13 @@ static int64_t registry_add(LineRegistry& r, uint64_t n) {
   int64_t idx = -1;
   std::unique_ptr<LenInfo> li(new LenInfo());
   const size_t cta_cap = 44 * 1024;  // the batch kernels' four-CTA share of an SM
+  // (a registered length does not know how many lines will share a launch:
+  // half-size long tasks)
   if (n >= 2 && n <= 0xFFFFFFFFull && r.infos.size() < kRegLengths &&
       classify(n, r.direction, r.normalization, cta_cap, r.cl_cap, false, *li) &&
       li->d.kind != BK_CL_MIXED && li->d.kind != BK_CL_BLUE) {
+    if (li->d.kind == BK_LONG || li->d.kind == BK_LONG_BLUE)
+      set_long_tasks(li->lng, kLongTaskValues / 2);
     std::vector<cd> tw;
     length_twiddles(*li, tw, r.tw_used);
     bool ok = r.tw_used + tw.size() <= kRegTwiddles;
@@ -1322,12 +1464,16 @@ static int64_t registry_add(LineRegistry& r, uint64_t n) {
       li->d.bhat = (const c32*)p;
       li->lng.bhat = (const c32*)p;
     }
-    if (ok && !li->pin.empty()) {
-      void *a = nullptr, *b = nullptr;
-      ok = upload(li->pin.data(), li->pin.size() * 4, &a) &&
-           upload(li->pout.data(), li->pout.size() * 4, &b);
-      li->d.perm_in = (const uint32_t*)a;
-      li->d.perm_out = (const uint32_t*)b;
+    if (ok && !li->perm.empty()) {
+      void* a = nullptr;
+      ok = upload(li->perm.data(), li->perm.size() * 4, &a);
+      li->d.perm = (const uint32_t*)a;
+    }
+    if (ok && !li->chirp.empty()) {
+      const std::vector<float> f = pack_f32(li->chirp);
+      void* a = nullptr;
+      ok = upload(f.data(), f.size() * 4, &a);
+      li->d.chirp = (const c32*)a;
     }
     if (ok) {
       idx = (int64_t)r.infos.size();
@@ -1393,14 +1539,17 @@ b2f_status line_batch_run(LineRegistry* reg, cudaStream_t st, const uint64_t* le
   std::vector<uint64_t> off_in, off_out;
   std::vector<LongTask> lt[3];
   uint64_t scratch = 0;
-  uint32_t buf_cta = 1, long_cap = 0;
+  uint32_t buf_cta = 1, long_cap = 0, long_tab = 0;
   for (auto& kv : by_idx) {
     const LenInfo& li = *reg->infos[kv.first];
     const BatchLen& d = li.d;
     if (d.kind == BK_LONG || d.kind == BK_LONG_BLUE) {
       const LongLenDesc& g = li.lng;
-      const uint32_t Gc = 1u << g.lgc, Gr = 1u << g.lgr;
-      long_cap = std::max(long_cap, std::max(g.N1 * (Gc + 1), g.N2 * (Gr + 1)));
+      const uint32_t Gc = g.c.G, Gr = g.r.G;
+      for (int ph = 1; ph <= 3; ++ph) {
+        long_cap = std::max(long_cap, long_task_values(g, ph));
+        long_tab = std::max(long_tab, long_table_values(g, ph));
+      }
       for (uint64_t line : kv.second) {
         const uint64_t sc = scratch;
         scratch += g.M;
@@ -1414,7 +1563,7 @@ b2f_status line_batch_run(LineRegistry* reg, cudaStream_t st, const uint64_t* le
       }
       continue;
     }
-    buf_cta = std::max<uint32_t>(buf_cta, d.G * d.LD);
+    buf_cta = std::max<uint32_t>(buf_cta, cta_task_values(d));
     const uint32_t first = (uint32_t)off_in.size();
     for (uint64_t line : kv.second) {
       off_in.push_back(in_off[line]);
@@ -1479,8 +1628,8 @@ b2f_status line_batch_run(LineRegistry* reg, cudaStream_t st, const uint64_t* le
   if (e == cudaSuccess && nlt)
     e = cudaMemcpyAsync(d_lt, lt_all.data(), nlt * sizeof(LongTask), cudaMemcpyHostToDevice, st);
   // the kernels' shared-memory limits, raised to the largest seen so far
-  const size_t smem_cta = 2 * (size_t)buf_cta * 8 + 2 * kBatchMaxG * 8;
-  const size_t smem_long = (3 * (size_t)long_cap + 2 * kLongTab) * 8;
+  const size_t smem_cta = (size_t)buf_cta * 8;
+  const size_t smem_long = ((size_t)long_cap + long_tab) * 8;
   if (e == cudaSuccess && !cta.empty() && smem_cta > reg->cta_smem_set) {
     e = set_smem(k_batch_cta, smem_cta);
     reg->cta_smem_set = smem_cta;
@@ -1530,7 +1679,7 @@ b2f_status line_batch_run(LineRegistry* reg, cudaStream_t st, const uint64_t* le
         lp.counter = counters + 4 + ph;
         const unsigned grid = (unsigned)std::min<uint64_t>(
             (uint64_t)reg->nsm * std::max(reg->long_per_sm, 1), (count + kLongChunk - 1) / kLongChunk);
-        if (ph == 0) k_long_pass<1><<<grid, kLongThreads, smem_long, st>>>(lp);
+          if (ph == 0) k_long_pass<1><<<grid, kLongThreads, smem_long, st>>>(lp);
         else if (ph == 1) k_long_pass<2><<<grid, kLongThreads, smem_long, st>>>(lp);
         else k_long_pass<3><<<grid, kLongThreads, smem_long, st>>>(lp);
         e = cudaGetLastError();

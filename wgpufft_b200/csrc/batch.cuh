@@ -3,7 +3,8 @@
 // Persistent kernels share one execute call:
 //  - k_batch_cta: each CTA repeatedly takes the next task from an atomic
 //    counter; a task is up to G lines of one length whose FFT (mixed radix,
-//    Rader or Bluestein) fits one CTA's shared memory;
+//    Rader or Bluestein, on the in-place stages of ipfft.cuh) fits one CTA's
+//    share of the shared memory;
 //  - k_long_pass (longpass.cuh): the longer lines, as column and row passes
 //    through a scratch region;
 //  - k_batch_cluster<P> (optional route for the longer lines): a thread-block cluster of P CTAs takes one long line
@@ -23,7 +24,7 @@
 #pragma once
 #include <cooperative_groups.h>
 
-#include "kernels_impl.cuh"
+#include "ipfft.cuh"
 
 namespace b2f {
 
@@ -37,24 +38,33 @@ enum BatchKind : uint32_t {
   BK_LONG_BLUE = 6, // long Bluestein line: three passes over M = N1*N2 (k_long_pass)
 };
 
+// What the in-place stages (Ip) read of a schedule: rows of one line or of
+// several, or adjacent columns.
+struct IpRows {
+  IpSched sc;
+  uint32_t G, lam, pitch, LDl, flags;
+  FastDiv dlam, dG;
+};
+
 struct BatchLen {
   uint32_t kind;
   uint32_t N;     // line length
   uint32_t M;     // transform length: N, p-1, or the convolution length
   uint32_t G;     // lines per task (CTA kinds)
-  uint32_t LD;    // shared-memory line pitch
+  uint32_t LD;    // shared-memory line pitch (cluster kinds, lines of up to 16 points)
   uint32_t P;     // cluster ranks in use (cluster kinds)
   uint32_t L;     // M / P (cluster kinds)
   float scale;    // normalisation of this length (f32, as the reference)
-  const c32* bhat;
-  const uint32_t* perm_in;
-  const uint32_t* perm_out;
-  FastDiv dN, dM, dMN, dP1;
+  const c32* bhat;        // [pos][k0] (CTA kinds), natural (cluster kinds)
+  const uint32_t* perm;   // Rader: g^q mod p
+  const c32* chirp;       // CTA Bluestein: exp(-i pi n^2 / N)
+  FastDiv dN;
   // two-level table of the cross-CTA twiddle W_M^j of the cluster kinds,
   // j = a*L + b (offsets into BatchParams::tw): ta[a] = W_M^{a L}, tb[b] = W_M^b.
   uint32_t ta, tb;
   FastDiv dB;
-  Schedule sch;   // schedule of the per-CTA FFT length (N, p-1, M or L)
+  IpRows ip;      // CTA kinds above 16 points: the transform of length M on G lines
+  Schedule sch;   // ping-pong schedule (cluster kinds: length L; lines of up to 16 points: N)
 };
 
 struct BatchTask {
@@ -104,22 +114,111 @@ FFT_D c32 tw2(const BatchParams& bp, const BatchLen& L, uint32_t j, uint32_t B) 
 }
 
 // --------------------------------------------------------------- CTA tasks
-FFT_D void batch_mixed(const BatchParams& bp, const BatchLen& L, const int64_t* base, const int64_t* obase, uint32_t cnt,
-                       c32* A, c32* B, uint32_t tid, uint32_t T) {
+// Global memory ends of the in-place stages: line g at base[g].
+struct BatchLoad {
+  const c32* in;
+  const int64_t* base;
+  bool cj;
+  template <int R>
+  FFT_D void load(c32* v, uint32_t g, uint32_t i, uint32_t step) const {
+    const c32* a = in + base[g] + i;
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = a[q * step];
+    if (cj) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q].im = -v[q].im;
+    }
+  }
+};
+
+struct BatchStore {
+  c32* out;
+  const int64_t* base;
+  float sc, sci;  // sci: scale of the imaginary part, negated for inverse transforms
+  template <int R>
+  FFT_D void store(c32* v, uint32_t g, uint32_t k, uint32_t step) const {
+    c32* a = out + base[g] + k;
+#pragma unroll
+    for (int q = 0; q < R; ++q) a[q * step] = c32{v[q].re * sc, v[q].im * sci};
+  }
+};
+
+struct BatchScatter {  // Rader: conv = conj(v) at r -> point g^-r of the staged line
+  c32* stage;
+  const uint32_t* perm;
+  uint32_t n;
+  template <int R>
+  FFT_D void store(c32* v, uint32_t g, uint32_t r, uint32_t step) const {
+    uint32_t j[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const uint32_t rr = r + q * step;
+      j[q] = __ldg(perm + (rr ? n - 1 - rr : 0));
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) stage[g * n + j[q]] = conj(v[q]);
+  }
+};
+
+struct BatchChirpLoad {
+  const c32* in;
+  const int64_t* base;
+  const c32* chirp;
+  uint32_t n;
+  bool cj;
+  template <int R>
+  FFT_D void load(c32* v, uint32_t g, uint32_t i, uint32_t step) const {
+    const c32* a = in + base[g];
+    constexpr int H = (R + 1) / 2;  // as IpChirpLoad
+    c32 w[H];
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = czero<float>();
+#pragma unroll
+    for (int q = 0; q < H; ++q) {
+      w[q] = czero<float>();
+      if (i + q * step < n) {
+        v[q] = a[i + q * step];
+        w[q] = chirp[i + q * step];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < H; ++q) {
+      if (cj) v[q].im = -v[q].im;
+      if (i + q * step < n) v[q] = cmul(v[q], w[q]);
+    }
+  }
+};
+
+struct BatchChirpStore {
+  c32* out;
+  const int64_t* base;
+  const c32* chirp;
+  uint32_t n;
+  float sc, sci;
+  template <int R>
+  FFT_D void store(c32* v, uint32_t g, uint32_t k, uint32_t step) const {
+    c32* a = out + base[g];
+    constexpr int H = (R + 1) / 2;
+#pragma unroll
+    for (int q = 0; q < H; ++q)
+      if (k + q * step < n) {
+        const c32 x = cmul(conj(v[q]), chirp[k + q * step]);
+        a[k + q * step] = c32{x.re * sc, x.im * sci};
+      }
+  }
+};
+
+// Lines of up to 16 points: one or two ping-pong stages.
+FFT_D void batch_tiny(const BatchParams& bp, const BatchLen& L, const int64_t* base,
+                      const int64_t* obase, uint32_t cnt, c32* A, c32* B, uint32_t tid, uint32_t T) {
   constexpr int PAD = PadOf<float>::value;
   const uint32_t N = L.N, LD = L.LD;
   const bool inv = bp.inverse;
   for (uint32_t e = tid; e < cnt * N; e += T) {
     const uint32_t c = fdiv(e, L.dN), n = e - c * N;
-    cp_async8(&A[c * LD + pidx<PAD>(n)], &bp.in[base[c] + n]);
-  }
-  cp_async_wait_all();
-  if (inv) {
-    for (uint32_t e = tid; e < cnt * N; e += T) {
-      const uint32_t c = fdiv(e, L.dN), n = e - c * N;
-      c32& v = A[c * LD + pidx<PAD>(n)];
-      v.im = -v.im;
-    }
+    c32 v = bp.in[base[c] + n];
+    if (inv) v.im = -v.im;
+    A[c * LD + pidx<PAD>(n)] = v;
   }
   __syncthreads();
   const c32* r = fft_lines_smem<float>(A, B, L.sch, cnt, LD, tid, T, bp.tw);
@@ -133,93 +232,73 @@ FFT_D void batch_mixed(const BatchParams& bp, const BatchLen& L, const int64_t* 
   }
 }
 
-FFT_D void batch_rader(const BatchParams& bp, const BatchLen& L, const int64_t* base, const int64_t* obase, uint32_t cnt,
-                       c32* A, c32* B, c32* x0s, c32* X0s, uint32_t tid, uint32_t T) {
-  constexpr int PAD = PadOf<float>::value;
-  const uint32_t P = L.N, P1 = L.M, LD = L.LD;
+// The task's lines on the in-place stages; `buf`: cnt * LDl values of data,
+// then for Rader the staged lines and x[0], X[0] of each.
+FFT_D void batch_lines(const BatchParams& bp, const BatchLen& L, const int64_t* base,
+                       const int64_t* obase, uint32_t cnt, c32* buf, uint32_t tid, uint32_t T) {
   const bool inv = bp.inverse;
-  for (uint32_t e = tid; e < cnt * P; e += T) {
-    const uint32_t c = fdiv(e, L.dN), n = e - c * P;
-    c32 v = bp.in[base[c] + n];
-    if (inv) v.im = -v.im;
-    A[c * LD + pidx<PAD>(n)] = v;
-  }
-  __syncthreads();
-  if (tid < cnt) x0s[tid] = A[tid * LD];
-  for (uint32_t e = tid; e < cnt * P1; e += T) {
-    const uint32_t l = fdiv(e, L.dP1), q = e - l * P1;
-    B[l * LD + pidx<PAD>(q)] = A[l * LD + pidx<PAD>(L.perm_in[q])];
-  }
-  __syncthreads();
-  c32* r1 = fft_lines_smem<float>(B, A, L.sch, cnt, LD, tid, T, bp.tw);
-  c32* o1 = (r1 == A) ? B : A;
-  if (tid < cnt) X0s[tid] = x0s[tid] + r1[tid * LD];
-  __syncthreads();
-  for (uint32_t e = tid; e < cnt * P1; e += T) {
-    const uint32_t l = fdiv(e, L.dP1), m = e - l * P1;
-    c32 v = cmul(r1[l * LD + pidx<PAD>(m)], L.bhat[m]);
-    v.im = -v.im;
-    r1[l * LD + pidx<PAD>(m)] = v;
-  }
-  __syncthreads();
-  const c32* r2 = fft_lines_smem<float>(r1, o1, L.sch, cnt, LD, tid, T, bp.tw);
-  const float sc = L.scale;
-  for (uint32_t e = tid; e < cnt * P; e += T) {
-    const uint32_t c = fdiv(e, L.dN), n = e - c * P;
-    c32 v;
-    if (n == 0) {
-      v = X0s[c];
-    } else {
-      c32 w = r2[c * LD + pidx<PAD>(L.perm_out[n - 1])];
-      w.im = -w.im;
-      v = x0s[c] + w;
-    }
-    v.re *= sc;
-    v.im = inv ? -v.im * sc : v.im * sc;
-    bp.out[obase[c] + n] = v;
-  }
-}
-
-FFT_D void batch_blue(const BatchParams& bp, const BatchLen& L, const int64_t* base, const int64_t* obase, uint32_t cnt,
-                      c32* A, c32* B, uint32_t tid, uint32_t T) {
-  constexpr int PAD = PadOf<float>::value;
-  const uint32_t N = L.N, M = L.M, LD = L.LD;
-  const bool inv = bp.inverse;
-  for (uint32_t e = tid; e < cnt * M; e += T) {
-    const uint32_t c = fdiv(e, L.dM), m = e - c * M;
-    c32 v = czero<float>();
-    if (m < N) {
-      v = bp.in[base[c] + m];
+  const float sc = L.scale, sci = inv ? -L.scale : L.scale;
+  const Ip<float, false, IpRows> ip{L.ip, buf, bp.tw, tid, T, cnt};
+  if (L.kind == BK_MIXED) {
+    ip.first(BatchLoad{bp.in, base, inv});
+    ip.forward_mids();
+    ip.last(BatchStore{bp.out, obase, sc, sci});
+  } else if (L.kind == BK_BLUE) {
+    ip.first(BatchChirpLoad{bp.in, base, L.chirp, L.N, inv});
+    ip.forward_mids();
+    ip.centre(IpConvOp<float>{L.bhat});
+    ip.inverse_mids();
+    ip.final_dit(BatchChirpStore{bp.out, obase, L.chirp, L.N, sc, sci});
+  } else {  // Rader
+    const uint32_t n = L.N;
+    c32* stage = buf + cnt * L.ip.LDl;
+    c32* x0 = stage + cnt * n;
+    c32* X0 = x0 + cnt;
+    for (uint32_t e = tid; e < cnt * n; e += T) {
+      const uint32_t c = fdiv(e, L.dN), i = e - c * n;
+      c32 v = bp.in[base[c] + i];
       if (inv) v.im = -v.im;
-      v = cmul(v, chirp<float>(m, N));
+      stage[e] = v;
+      if (i == 0) x0[c] = v;
     }
-    A[c * LD + pidx<PAD>(m)] = v;
-  }
-  __syncthreads();
-  c32* r1 = fft_lines_smem<float>(A, B, L.sch, cnt, LD, tid, T, bp.tw);
-  c32* o1 = (r1 == A) ? B : A;
-  for (uint32_t e = tid; e < cnt * M; e += T) {
-    const uint32_t l = fdiv(e, L.dM), m = e - l * M;
-    c32 v = cmul(r1[l * LD + pidx<PAD>(m)], L.bhat[m]);
-    v.im = -v.im;
-    r1[l * LD + pidx<PAD>(m)] = v;
-  }
-  __syncthreads();
-  const c32* r2 = fft_lines_smem<float>(r1, o1, L.sch, cnt, LD, tid, T, bp.tw);
-  const float sc = L.scale;
-  for (uint32_t e = tid; e < cnt * N; e += T) {
-    const uint32_t c = fdiv(e, L.dN), k = e - c * N;
-    c32 w = r2[c * LD + pidx<PAD>(k)];
-    w.im = -w.im;
-    c32 v = cmul(w, chirp<float>(k, N));
-    v.re *= sc;
-    v.im = inv ? -v.im * sc : v.im * sc;
-    bp.out[obase[c] + k] = v;
+    __syncthreads();
+    ip.first(IpGather<float, false>{stage, L.perm, n, 0});
+    ip.forward_mids();
+    ip.centre(IpRaderOp<float>{L.bhat, x0, X0});
+    ip.inverse_mids();
+    ip.final_dit(BatchScatter{stage, L.perm, n});
+    for (uint32_t c = tid; c < cnt; c += T) stage[c * n] = X0[c];
+    __syncthreads();
+    for (uint32_t e = tid; e < cnt * n; e += T) {
+      const uint32_t c = fdiv(e, L.dN);
+      const c32 v = stage[e];
+      bp.out[obase[c] + (e - c * n)] = c32{v.re * sc, v.im * sci};
+    }
   }
 }
 
-// Persistent CTA kernel: blockDim.x threads, dynamic shared memory holds the
-// two line buffers of the largest task plus Rader's x0/X0 slots.
+// make_fastdiv for d < 2^16 on the device (the sub-lines of a task vary with
+// its line count).
+FFT_D FastDiv fastdiv_small(uint32_t d) {
+  FastDiv f;
+  f.d = d;
+  const uint32_t l = d > 1 ? 32 - __clz(d - 1) : 0;
+  if ((d & (d - 1)) == 0) {
+    f.mul = 0;
+    f.shift = l;
+  } else {
+    f.mul = (uint32_t)(((1ull << (31 + l)) + d - 1) / d);
+    f.shift = l - 1;
+  }
+  return f;
+}
+
+// Persistent CTA kernel: 256 threads, four CTAs an SM; dynamic shared memory
+// holds the largest task.  Issue-bound; with padded addresses, chirps and
+// their 64-bit modulos recomputed per point the short lines took 317 thread
+// instructions a point and Bluestein lines above 1,400 points the three-pass
+// route: 964 lines of up to 2,293 points 95 -> 31 us, 1,300 of up to 1,849
+// 91 -> 26 us.
 __global__ void __launch_bounds__(256, 4) k_batch_cta(const __grid_constant__ BatchParams bp,
                                                    uint32_t buf_elems) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -229,13 +308,10 @@ __global__ void __launch_bounds__(256, 4) k_batch_cta(const __grid_constant__ Ba
   __shared__ uint32_t s_task;
   uint32_t s_len_idx = 0xFFFFFFFFu;  // length descriptor currently in s_len (same in every thread)
   c32* A = reinterpret_cast<c32*>(smem_raw);
-  c32* B = A + buf_elems;
-  c32* x0s = B + buf_elems;
-  c32* X0s = x0s + kBatchMaxG;
   const uint32_t tid = threadIdx.x, T = blockDim.x;
+  if (tid == 0) s_task = atomicAdd(bp.counter, 1u);
+  __syncthreads();
   for (;;) {
-    if (tid == 0) s_task = atomicAdd(bp.counter, 1u);
-    __syncthreads();
     const uint32_t t = s_task;
     if (t >= bp.ntasks) break;
     const BatchTask task = bp.tasks[t];
@@ -245,15 +321,22 @@ __global__ void __launch_bounds__(256, 4) k_batch_cta(const __grid_constant__ Ba
       s_base[c] = (int64_t)bp.line_off[task.first + c];
       s_obase[c] = (int64_t)(bp.line_off_out ? bp.line_off_out : bp.line_off)[task.first + c];
     }
-    __syncthreads();
-    switch (s_len.kind) {
-      case BK_MIXED: batch_mixed(bp, s_len, s_base, s_obase, task.count, A, B, tid, T); break;
-      case BK_RADER:
-        batch_rader(bp, s_len, s_base, s_obase, task.count, A, B, x0s, X0s, tid, T);
-        break;
-      case BK_BLUE: batch_blue(bp, s_len, s_base, s_obase, task.count, A, B, tid, T); break;
-      default: break;
+    __syncthreads();  // s_task read, s_len and the line offsets written
+    uint32_t next = 0;
+    if (tid == 0) {
+      next = atomicAdd(bp.counter, 1u);
+      if (s_len.ip.sc.N) {  // the sub-lines of this task's lines
+        const uint32_t lam = task.count * s_len.ip.sc.R0;
+        s_len.ip.lam = lam;
+        s_len.ip.dlam = fastdiv_small(lam);
+      }
     }
+    __syncthreads();
+    if (s_len.ip.sc.N)
+      batch_lines(bp, s_len, s_base, s_obase, task.count, A, tid, T);
+    else
+      batch_tiny(bp, s_len, s_base, s_obase, task.count, A, A + buf_elems / 2, tid, T);
+    if (tid == 0) s_task = next;
     __syncthreads();
   }
 }

@@ -85,10 +85,11 @@ FFT_D void ip_radix(uint32_t R, F f) {
   }
 }
 
-// The lines of one CTA in shared memory.
-template <class S, bool COL>
+// The lines of one CTA in shared memory; P: IpParams, or the part of it
+// that the stages read (sc, G, lam, pitch, LDl, flags, dlam, dG).
+template <class S, bool COL, class P = IpParams>
 struct Ip {
-  const IpParams& p;
+  const P& p;
   C<S>* sm;
   const C<S>* tw;
   uint32_t tid, T, nvalid;
@@ -288,11 +289,11 @@ struct Ip {
   }
 
   // A convolution's centre: last forward stage, product with the spectrum
-  // (op.dc sees frequency 0 first), conjugate, first inverse stage.
+  // (op.spectrum(g), [pos][k0]; op.dc sees frequency 0 first), conjugate,
+  // first inverse stage.
   template <class Op>
   FFT_D void centre(const Op& op) const {
     const IpStage& s = p.sc.st[p.sc.nst - 1];
-    const C<S>* __restrict__ bhat = (const C<S>*)p.bhat;
     const uint32_t R0 = COL ? 1u : p.sc.R0;
     ip_radix(s.R, [&](auto rc) {
       constexpr int R = decltype(rc)::value;
@@ -305,7 +306,7 @@ struct Ip {
 #pragma unroll
         for (int q = 0; q < R; ++q) v[q] = a[q * is()];
         dft<S, R>(v);
-        const C<S>* w = bhat + (b * R) * R0 + k0;
+        const C<S>* __restrict__ w = op.spectrum(g) + (b * R) * R0 + k0;
         const C<S> v0 = v[0];
 #pragma unroll
         for (int q = 0; q < R; ++q) v[q] = conj(cmul(v[q], w[q * R0]));
@@ -464,9 +465,11 @@ struct IpScatter {  // conv = conj(v) at r -> point g^-r
 };
 
 template <class S>
-struct IpRaderDc {
+struct IpRaderOp {
+  const C<S>* bhat;
   const C<S>* x0;
   C<S>* X0;
+  FFT_D const C<S>* spectrum(uint32_t) const { return bhat; }
   // X[0] = x[0] + A[0]; the product's conjugate gets conj(x[0])
   FFT_D void dc(uint32_t g, C<S> a0, C<S>& prod) const {
     const C<S> x = x0[g];
@@ -504,7 +507,7 @@ __global__ void __launch_bounds__(IpBounds<S>::threads)
   __syncthreads();
   ip.first(IpGather<S, COL>{stage, p.perm, n, G});
   ip.forward_mids();
-  ip.centre(IpRaderDc<S>{x0, X0});
+  ip.centre(IpRaderOp<S>{(const C<S>*)p.bhat, x0, X0});
   ip.inverse_mids();
   const S sc = Scalar<S>::from_double(p.scale);
   C<S>* out = (C<S>*)p.out + g.out0;
@@ -590,7 +593,9 @@ struct IpChirpStore {
 };
 
 template <class S>
-struct IpNoDc {
+struct IpConvOp {
+  const C<S>* bhat;
+  FFT_D const C<S>* spectrum(uint32_t) const { return bhat; }
   FFT_D void dc(uint32_t, C<S>, C<S>&) const {}
 };
 
@@ -604,7 +609,7 @@ __global__ void __launch_bounds__(IpBounds<S>::threads)
   const C<S>* chirp = (const C<S>*)p.chirp;
   ip.first(IpChirpLoad<S>{(const C<S>*)p.in + g.in0, chirp, g.dl_in, p.io.in_es, p.n, p.flags});
   ip.forward_mids();
-  ip.centre(IpNoDc<S>());
+  ip.centre(IpConvOp<S>{(const C<S>*)p.bhat});
   ip.inverse_mids();
   ip.final_dit(IpChirpStore<S>{(C<S>*)p.out + g.out0, chirp, g.dl_out, p.io.out_es, p.n,
                                    p.flags, Scalar<S>::from_double(p.scale)});

@@ -6,50 +6,49 @@
 //                W_T^{n2 k1}, into the scratch row k1 (natural [k1][n2]);
 //   row pass:    for each k1, FFT_N2 over n2 of scratch row k1, giving
 //                X[k1 + N1 k2].
-// A task is G (16, 8 or 4) adjacent columns or rows of one line, so every
-// global access is a segment of G consecutive complex values (128 bytes at
-// G = 16): rows of columns n2..n2+G-1, or the outputs k1..k1+G-1 of one k2.
-// The G lines of a task sit interleaved in shared memory, element (i, l) at
-// i*(G+1) + l: the 16 threads of a half-warp take the same position i of 16
-// lines, so the Stockham stages and the column segments are conflict-free,
-// and the pitch G+1 keeps the transposed row loads (consecutive i, fixed l)
-// conflict-free too.  Each thread keeps one line l and walks the butterflies
-// j = s, s+S, ... of every stage with incrementally updated offsets.
+// A task is G adjacent columns or rows of one line (up to 4,384 values), on
+// the in-place stages of ipfft.cuh: columns interleaved, first stage from
+// and last stage to global memory in segments of G values; rows with a lead
+// stage along the row, the last stage storing G adjacent rows' outputs
+// together.
 //
 // Bluestein lines (convolution M = N1 N2) take three passes: the chirped
 // column pass; a middle row pass that runs the forward row FFT, multiplies
 // by the chirp spectrum, and runs the row half of the inverse FFT
 // (y[N2 n1 + n2] = sum_k1 W_N1^{-n1 k1} W_M^{-n2 k1} sum_k2 W_N2^{-n2 k2} Y[k1 + N1 k2],
-// computed on conjugates with the forward codelets) in place on the rows;
-// and the inverse column pass, chirped into the output.  One scratch region
-// of M values per line.
+// computed on conjugates with the forward codelets) in place on the rows,
+// never leaving the digit-reversed order in between; and the inverse column
+// pass, chirped into the output.  One scratch region of M values per line.
 //
-// Loads are asynchronous (cp.async): while a CTA transforms one task, the
-// copies of its next task are already in flight into the other landing
-// buffer, together with the twiddle tables of its length (stage twiddles,
-// W_M^{a N2} and W_M^b) when they differ from the ones that buffer last
-// held.  The work queue hands out chunks of consecutive tasks (mostly one
-// line), so the tables change rarely; nothing waits on another CTA.
+// The work queue hands out chunks of consecutive tasks (mostly one line); a
+// task's record and length descriptor arrive by asynchronous copies two and
+// three tasks ahead, the two-level tables of its length (W_M, and the
+// chirp) when they differ from the last task's.  The data itself is not
+// prefetched: four CTAs of 256 threads and 64 registers share an SM and
+// cover each other's loads (fetching the next task's data or tables into L2
+// ahead cost its instructions and 3 % instead).
+//
+// What bounds it: instruction issue, 335 thread instructions per point of
+// the 20,000-line mixed workload (540 with the earlier ping-pong stages and
+// 16 warps an SM) at 44-50 % of the issue slots, behind loads, barriers and,
+// as neighbouring tasks run other radices, instruction fetch.  That workload:
+// 4.32 -> 3.14 ms; 512 x 65536: 404 -> 244 us; 512 x 65521 (Bluestein): 1994
+// -> 1026; 1118 x 30011: 1676 -> 853; 6706 x 5003: 2122 -> 931.
 #pragma once
 #include "batch.cuh"
+#include "ipfft.cuh"
 
 namespace b2f {
 
 constexpr uint32_t kLongThreads = 256;
-constexpr uint32_t kLongThreadsLog2 = 8;
-static_assert(kLongThreads == 1u << kLongThreadsLog2, "thread count is a power of two");
-constexpr int kLongMaxStages = 10;  // pass lengths <= 512
 constexpr uint32_t kLongChunk = 4;  // consecutive tasks per work-queue claim
 // k_long_pass claims the first two chunks before its loop and every later
 // one when the chunk before it opens (three tasks ahead): that covers every
 // chunk only when a chunk holds at least three tasks
 static_assert(kLongChunk >= 3, "the prologue claims chunks 0 and 1 only");
-// table area of one landing buffer (complex values): stage twiddles of the
-// pass (length - 1 <= 511), W_M^{a N2} (a < N1 <= 512), W_M^b (b < N2 <= 512);
-// the Bluestein inverse column pass holds the chirp tables W_2N^{a B} and
-// W_2N^b (B = ceil(sqrt(2N)) <= 512) where the last two are
-constexpr uint32_t kTabSt = 0, kTabTa = 512, kTabTb = 1024;
-constexpr uint32_t kLongTab = 1536;
+// Values a task holds in shared memory: sixteen columns of 272 points or rows of 256.  With
+// the tables (at most 2048 values) four CTAs share an SM.
+constexpr uint32_t kLongTaskValues = 4384;
 
 enum LongPassKind : uint32_t {
   LP_COL = 0,    // smooth line, column pass: x -> scratch
@@ -59,24 +58,20 @@ enum LongPassKind : uint32_t {
   LP_BCOL3 = 4,  // Bluestein, inverse column pass, chirped: scratch -> out
 };
 
-struct LongSched {
-  uint32_t nst;
-  StageDesc st[kLongMaxStages];
-};
-
 struct LongLenDesc {
   uint32_t N, M, N1, N2;
-  uint32_t lgc, lgr;  // log2 of the lines per column / row task
   uint32_t blue;
   float scale;
-  const c32* bhat;    // Bluestein: spectrum of the conjugate chirp / M, natural order
+  const c32* bhat;  // Bluestein: spectrum of the conjugate chirp / M, row k1 at k1 * N2 in the
+                    // order the row's frequencies take ([pos][k0])
   // two-level tables (offsets into the twiddle table) with rows of
   // L = 2^tsplit >= sqrt(M): W_M^j = W_M^{L a} * W_M^b, j = a L + b,
-  // a < ceil(M / L) <= 512, b < L <= 512; the Bluestein chirp W_2N^q
+  // a < tn = ceil(M / L) <= 512, b < L <= 512; the Bluestein chirp W_2N^q
   // likewise with rows of 2^csplit >= sqrt(2N)
-  uint32_t ta, tb, tsplit;
-  uint32_t ca, cb, csplit;
-  LongSched s1, s2;   // schedules of N1 (columns) and N2 (rows)
+  uint32_t ta, tb, tn, tsplit;
+  uint32_t ca, cb, cn, csplit;
+  uint32_t minv, mshift;  // n^2 mod 2N (mod_square)
+  IpRows c, r;            // columns of N1, rows of N2
 };
 
 // One task: G adjacent columns or rows of one line.  Self-contained, so
@@ -101,7 +96,7 @@ struct LongParams {
   uint32_t ntasks;
   uint32_t phase;    // 1: column pass, 2: row pass, 3: Bluestein inverse columns
   uint32_t inverse;
-  uint32_t cap;      // complex elements per shared-memory buffer
+  uint32_t cap;      // complex elements of the data buffer
   unsigned int* counter;  // work queue: chunks of kLongChunk tasks handed out in order
 };
 
@@ -111,456 +106,248 @@ FFT_D void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-FFT_D uint32_t long_kind(uint32_t phase, bool blue) {
-  if (phase == 1) return blue ? LP_BCOL1 : LP_COL;
-  if (phase == 2) return blue ? LP_BMID : LP_ROW;
-  return LP_BCOL3;
-}
-
-// W^j from a two-level table with rows of 2^sh: j = a*2^sh + b, value
-// ta[a] * tb[b] (a shift and a mask, no division).
-FFT_D c32 tw_two(const c32* __restrict__ tw, uint32_t ta, uint32_t tb, uint32_t j, uint32_t sh) {
-  return cmul(tw[ta + (j >> sh)], tw[tb + (j & ((1u << sh) - 1))]);
-}
-
-// Where the last stage of a pass puts its results: back into shared memory
-// (EpiNone), or straight from registers to global memory, the R outputs
-// v[r] of one butterfly of line l at positions o + r*Ns: the column pass's
-// scratch store with the inter-pass twiddle (EpiCol), the row pass's output
-// store (EpiRow).  Addresses and twiddle exponents advance by a fixed step
-// per output.  A half-warp holds one position of 16 lines, so each store is
-// one G-value segment.
-struct EpiNone {
-  static constexpr bool active = false;
-  template <int R>
-  FFT_D void store(uint32_t, uint32_t, const c32*) const {}
+// W^j from a two-level table in shared memory (a shift and a mask).
+struct TwoLevel {
+  const c32* hi;
+  const c32* lo;
+  uint32_t sh;
+  FFT_D c32 at(uint32_t j) const { return cmul(hi[j >> sh], lo[j & ((1u << sh) - 1)]); }
 };
-struct EpiCol {  // scratch[N2 pos + c] = v * W_M^{c pos}
-  static constexpr bool active = true;
-  c32* dst;  // scratch of the line + c
-  const c32* T;
-  uint32_t N2, c, sh;
-  bool ok;
+
+// n^2 mod m for n < 2^17, m = 2N < 2^19: the quotient estimate is
+// umulhi(n^2 / 4, minv) >> mshift with minv = (2^(32+b) - 1) / m, 2^b <= m <
+// 2^(b+1), mshift = b - 2.  Before the shift it is short by less than 3
+// (the two dropped bits, minv's and umulhi's truncation), so after it by at
+// most 1 when 2^mshift >= 3: one conditional subtraction.
+FFT_D uint32_t mod_square(uint32_t n, uint32_t m, uint32_t minv, uint32_t mshift) {
+  const uint64_t sq = (uint64_t)n * n;
+  const uint32_t q = __umulhi((uint32_t)(sq >> 2), minv) >> mshift;
+  const uint32_t r = (uint32_t)sq - q * m;
+  return r >= m ? r - m : r;
+}
+
+// The chirp exp(-i pi n^2 / N).
+struct LongChirp {
+  TwoLevel t;
+  uint32_t N, minv, mshift;
+  FFT_D c32 at(uint32_t n) const { return t.at(mod_square(n, 2 * N, minv, mshift)); }
+};
+
+// ---- global memory ends; g counts the task's columns or rows
+struct LongColLoad {  // point i of column g at src[N2 i + g]
+  const c32* src;
+  uint32_t N2;
+  bool cj;
   template <int R>
-  FFT_D void store(uint32_t o, uint32_t Ns, const c32* v) const {
-    if (!ok) return;
-    uint32_t e = c * o;  // c * pos < M
-    const uint32_t de = c * Ns;
-    c32* dp = dst + (uint64_t)N2 * o;
-    const uint64_t step = (uint64_t)N2 * Ns;
+  FFT_D void load(c32* v, uint32_t g, uint32_t i, uint32_t step) const {
+    const c32* a = src + (uint64_t)N2 * i + g;
+    const uint64_t d = (uint64_t)N2 * step;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      *dp = cmul(v[r], tw_two(T, kTabTa, kTabTb, e, sh));
+    for (int q = 0; q < R; ++q) v[q] = a[q * d];
+    if (cj) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q].im = -v[q].im;
+    }
+  }
+};
+
+struct LongChirpLoad {  // the same of the chirped, zero-padded line; c0: first column
+  const c32* src;
+  LongChirp ch;
+  uint32_t N2, c0;
+  bool cj;
+  template <int R>
+  FFT_D void load(c32* v, uint32_t g, uint32_t i, uint32_t step) const {
+    const uint32_t n = N2 * i + c0 + g, dn = N2 * step;
+    // M >= 2N - 1: rows below N1 / 2 hold data, so the first half of a
+    // butterfly's points, rounded up
+    constexpr int H = (R + 1) / 2;
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = czero<float>();
+#pragma unroll
+    for (int q = 0; q < H; ++q)
+      if (n + q * dn < ch.N) v[q] = src[n + q * dn];
+#pragma unroll
+    for (int q = 0; q < H; ++q)
+      if (n + q * dn < ch.N) {
+        if (cj) v[q].im = -v[q].im;
+        v[q] = cmul(v[q], ch.at(n + q * dn));
+      }
+  }
+};
+
+struct LongColStore {  // scratch[N2 k + c] = v * W_M^{c k}
+  c32* dst;  // scratch + first column
+  TwoLevel t;
+  uint32_t N2, c0;
+  template <int R>
+  FFT_D void store(c32* v, uint32_t g, uint32_t k, uint32_t step) const {
+    const uint32_t c = c0 + g;
+    uint32_t e = c * k;  // c k < M
+    const uint32_t de = c * step;
+    c32* a = dst + (uint64_t)N2 * k + g;
+    const uint64_t d = (uint64_t)N2 * step;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      *a = cmul(v[q], t.at(e));
       e += de;
-      dp += step;
+      a += d;
     }
   }
 };
-struct EpiRow {  // out[k1 + N1 pos], scaled, conjugated back for inverse transforms
-  static constexpr bool active = true;
-  c32* dst;  // out of the line + k1
+
+struct LongRowStore {  // out[k1 + N1 k], scaled, conjugated back for inverse transforms
+  c32* dst;  // out + first row
   uint32_t N1;
-  float sc, sci;  // scale of the real and imaginary parts (sci = -sc for inverse)
-  bool ok;
+  float sc, sci;
   template <int R>
-  FFT_D void store(uint32_t o, uint32_t Ns, const c32* v) const {
-    if (!ok) return;
-    c32* dp = dst + (uint64_t)N1 * o;
-    const uint64_t step = (uint64_t)N1 * Ns;
+  FFT_D void store(c32* v, uint32_t g, uint32_t k, uint32_t step) const {
+    c32* a = dst + (uint64_t)N1 * k + g;
+    const uint64_t d = (uint64_t)N1 * step;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      *dp = c32{v[r].re * sc, v[r].im * sci};
-      dp += step;
+    for (int q = 0; q < R; ++q) {
+      *a = c32{v[q].re * sc, v[q].im * sci};
+      a += d;
     }
   }
 };
 
-// One radix-R stage over G interleaved lines, src -> dst (or, for the last
-// stage with an active epilogue, src -> epi): thread (l, s) runs the
-// butterflies j = s, s+S, ... of line l; k = j mod Ns advances by S mod Ns.
-// tws: this stage's twiddles, row k at k*(R-1).
-template <int R, class Epi>
-FFT_D void ilv_stage(const c32* __restrict__ src, c32* __restrict__ dst, const StageDesc& sd,
-                     uint32_t lg, uint32_t tid, const c32* __restrict__ tws, bool to_epi,
-                     const Epi& epi) {
-  const uint32_t G = 1u << lg, P = G + 1;
-  const uint32_t l = tid & (G - 1), s = tid >> lg, S = kLongThreads >> lg;
-  const uint32_t NR = sd.NR, Ns = sd.Ns;
-  if (s >= NR) return;
-  const uint32_t qs = NR * P, rs = Ns * P;
-  uint32_t k = 0, kinc = 0;
-  if (Ns > 1) {
-    k = s - fdiv(s, sd.dNs) * Ns;
-    kinc = S - fdiv(S, sd.dNs) * Ns;
+struct LongMidStore {  // scratch row k1, position i: v * W_M^{i k1}
+  c32* dst;  // scratch row of the task's first row
+  TwoLevel t;
+  uint32_t N2, k0;
+  template <int R>
+  FFT_D void store(c32* v, uint32_t g, uint32_t i, uint32_t step) const {
+    const uint32_t k1 = k0 + g;
+    uint32_t e = i * k1;
+    const uint32_t de = step * k1;
+    c32* a = dst + (uint64_t)N2 * g + i;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      a[q * step] = cmul(v[q], t.at(e));
+      e += de;
+    }
   }
-#pragma unroll(R <= 8 ? 2 : 1)
-  for (uint32_t j = s; j < NR; j += S) {
-    const c32* sb = src + j * P + l;
-    c32 v[R];
+};
+
+struct LongChirpStore {  // out[n] = conj(v) * chirp(n), n = N2 k + c < N
+  c32* dst;  // out
+  LongChirp ch;
+  uint32_t N2, c0;
+  float sc, sci;
+  template <int R>
+  FFT_D void store(c32* v, uint32_t g, uint32_t k, uint32_t step) const {
+    const uint32_t n0 = N2 * k + c0 + g, dn = N2 * step;
 #pragma unroll
-    for (int q = 0; q < R; ++q) v[q] = sb[q * qs];
-    if (Ns > 1) {
-      const c32* t = tws + k * (R - 1);
-#pragma unroll
-      for (int q = 1; q < R; ++q) v[q] = cmul(v[q], t[q - 1]);
+    for (int q = 0; q < R; ++q) {
+      const uint32_t n = n0 + q * dn;
+      if (n < ch.N) {
+        const c32 x = cmul(conj(v[q]), ch.at(n));
+        dst[n] = c32{x.re * sc, x.im * sci};
+      }
     }
-    dft<float, R>(v);
-    const uint32_t o = (j - k) * R + k;
-    if (Epi::active && to_epi) {
-      epi.template store<R>(o, Ns, v);
-    } else {
-      c32* db = dst + o * P + l;
-#pragma unroll
-      for (int r = 0; r < R; ++r) db[r * rs] = v[r];
-    }
-    k += kinc;
-    if (k >= Ns) k -= Ns;
+  }
+};
+
+struct LongConvOp {
+  const c32* bhat;  // spectrum of the task's first row
+  uint32_t N2;
+  FFT_D const c32* spectrum(uint32_t g) const { return bhat + (uint64_t)g * N2; }
+  FFT_D void dc(uint32_t, c32, c32&) const {}
+};
+
+FFT_D void long_copy(c32* dst, const c32* src, uint32_t n) {
+  for (uint32_t e = threadIdx.x; e < n; e += kLongThreads) cp_async8(dst + e, src + e);
+}
+
+// Issues the copies of a length's two-level tables that phase PH reads into
+// T: W_M at 0 and tn, the chirp behind it (or at 0 when the phase needs no
+// W_M).
+template <uint32_t PH>
+FFT_D void long_tables(const LongParams& p, const LongLenDesc& d, c32* T) {
+  if (PH != 3) {
+    long_copy(T, p.tw + d.ta, d.tn);
+    long_copy(T + d.tn, p.tw + d.tb, 1u << d.tsplit);
+    T += d.tn + (1u << d.tsplit);
+  }
+  if ((PH == 1 && d.blue) || PH == 3) {
+    long_copy(T, p.tw + d.ca, d.cn);
+    long_copy(T + d.cn, p.tw + d.cb, 1u << d.csplit);
   }
 }
 
-// The whole schedule, a <-> b; returns the buffer holding the result (with
-// an active epilogue the last stage goes to epi and the return value is
-// meaningless).  T: the table area (stage twiddles from offset kTabSt,
-// global table offsets relative to the first stage's).  The caller
-// synchronises before; every stage that writes shared memory ends with a
-// barrier.
-template <class Epi>
-FFT_D c32* ilv_fft(c32* a, c32* b, const LongSched& sch, uint32_t lg, uint32_t tid, const c32* T,
-                   const Epi& epi) {
-  const uint32_t tw0 = sch.st[0].tw_off;
-#pragma unroll 1
-  for (uint32_t s = 0; s < sch.nst; ++s) {
-    const StageDesc& sd = sch.st[s];
-    const c32* tws = T + kTabSt + (sd.tw_off - tw0);
-    const bool to_epi = Epi::active && s + 1 == sch.nst;
-    switch (sd.R) {
-      case 2: ilv_stage<2>(a, b, sd, lg, tid, tws, to_epi, epi); break;
-      case 3: ilv_stage<3>(a, b, sd, lg, tid, tws, to_epi, epi); break;
-      case 4: ilv_stage<4>(a, b, sd, lg, tid, tws, to_epi, epi); break;
-      case 5: ilv_stage<5>(a, b, sd, lg, tid, tws, to_epi, epi); break;
-      case 7: ilv_stage<7>(a, b, sd, lg, tid, tws, to_epi, epi); break;
-      case 8: ilv_stage<8>(a, b, sd, lg, tid, tws, to_epi, epi); break;
-      case 9: ilv_stage<9>(a, b, sd, lg, tid, tws, to_epi, epi); break;
-      case 11: ilv_stage<11>(a, b, sd, lg, tid, tws, to_epi, epi); break;
-      case 13: ilv_stage<13>(a, b, sd, lg, tid, tws, to_epi, epi); break;
-      case 16: ilv_stage<16>(a, b, sd, lg, tid, tws, to_epi, epi); break;
-      default: break;
-    }
-    if (to_epi) break;
+// One task of phase PH; the tables have been issued as a cp.async group of
+// their own when `fresh` (one younger group may be in flight).  The caller
+// synchronises before and after.
+template <uint32_t PH>
+FFT_D void long_task(const LongParams& p, const LongLenDesc& d, const LongTask& ln, c32* sm,
+                     const c32* T, bool fresh) {
+  const uint32_t tid = threadIdx.x, g0 = ln.g0;
+  const bool inv = p.inverse != 0;
+  const TwoLevel tw{T, T + d.tn, d.tsplit};
+  if (fresh && (PH == 1 && d.blue)) {  // the chirp tables serve the first loads
+    cp_async_wait<1>();
     __syncthreads();
-    c32* t = a;
-    a = b;
-    b = t;
+    fresh = false;
   }
-  return a;
-}
-
-// x mod m for x < 2^50, m < 2^32, inv = 1/m rounded to double: the
-// quotient estimate trunc(x * inv) is off by at most one (its relative
-// error is below 2^-51, x / m below 2^50), so one correction either way
-// gives the remainder.  A 64-bit integer modulo is a long software routine
-// on the GPU; this is a few instructions.
-FFT_D uint32_t mod_u50(uint64_t x, uint32_t m, double inv) {
-  const uint64_t q = (uint64_t)((double)x * inv);
-  int64_t r = (int64_t)x - (int64_t)(q * m);
-  if (r < 0) r += m;
-  else if (r >= (int64_t)m) r -= m;
-  return (uint32_t)r;
-}
-
-// Chirp exp(-i pi n^2 / N) at n, n + D, n + 2D, ... : q = n^2 mod 2N kept
-// incrementally ((n + D)^2 = n^2 + 2nD + D^2); W_2N^q from the length's
-// two-level chirp table (q = a B + b: ca[a] * cb[b]), read through the
-// read-only cache (value_ldg) or from a shared-memory copy (value).
-// n < 2^24 and D < 2^24 (the residues below need n^2, 2nD, 2D^2 < 2^50).
-struct ChirpWalk {
-  uint32_t q, u, dsq, u2, twoN, sh, mask;
-  const c32* ca;
-  const c32* cb;
-  FFT_D void init(uint64_t n, uint32_t D, uint32_t N, const c32* ta, const c32* tb,
-                  uint32_t split) {
-    ca = ta;
-    cb = tb;
-    sh = split;
-    mask = (1u << split) - 1;
-    twoN = 2 * N;
-    const double inv = 1.0 / (double)twoN;
-    q = mod_u50(n * n, twoN, inv);
-    u = mod_u50(2 * n * (uint64_t)D, twoN, inv);
-    dsq = mod_u50((uint64_t)D * D, twoN, inv);
-    u2 = mod_u50(2 * (uint64_t)D * D, twoN, inv);
-  }
-  FFT_D void step() {
-    q += u;
-    if (q >= twoN) q -= twoN;
-    q += dsq;
-    if (q >= twoN) q -= twoN;
-    u += u2;
-    if (u >= twoN) u -= twoN;
-  }
-  FFT_D c32 value_ldg() const {
-    const float2 x = __ldg(reinterpret_cast<const float2*>(ca + (q >> sh)));
-    const float2 y = __ldg(reinterpret_cast<const float2*>(cb + (q & mask)));
-    return cmul(c32{x.x, x.y}, c32{y.x, y.y});
-  }
-  FFT_D c32 value() const { return cmul(ca[q >> sh], cb[q & mask]); }
-};
-
-FFT_D void copy_async(c32* dst, const c32* src, uint32_t n, uint32_t tid) {
-  for (uint32_t e = tid; e < n; e += kLongThreads) cp_async8(dst + e, src + e);
-}
-
-// Issues the copies of one task into the landing buffer X (zero-filled
-// where the task has no data) and, with tables, of its length's twiddle
-// tables into the table area T.
-FFT_D void long_issue(const LongParams& p, const LongLenDesc& d, const LongTask& ln, uint32_t kind,
-                      c32* X, c32* T, bool tables, uint32_t tid) {
-  const uint32_t g0 = ln.g0;
-  const bool colk = kind == LP_COL || kind == LP_BCOL1 || kind == LP_BCOL3;
-  if (tables) {
-    const LongSched& sch = colk ? d.s1 : d.s2;
-    const uint32_t nx = colk ? d.N1 : d.N2;
-    copy_async(T + kTabSt, p.tw + sch.st[0].tw_off, nx - 1, tid);
-    if (kind == LP_COL || kind == LP_BCOL1 || kind == LP_BMID) {
-      copy_async(T + kTabTa, p.tw + d.ta, (d.M + (1u << d.tsplit) - 1) >> d.tsplit, tid);
-      copy_async(T + kTabTb, p.tw + d.tb, 1u << d.tsplit, tid);
-    } else if (kind == LP_BCOL3) {
-      // the chirp tables (ceil(2N / B) <= B <= 512 values each) in their place
-      copy_async(T + kTabTa, p.tw + d.ca, (2 * d.N + (1u << d.csplit) - 1) >> d.csplit, tid);
-      copy_async(T + kTabTb, p.tw + d.cb, 1u << d.csplit, tid);
+  auto landed = [&] {
+    if (fresh) {
+      cp_async_wait<1>();
+      __syncthreads();
     }
-  }
-  if (colk) {
-    // columns g0..g0+G-1: row n1 is the segment src[N2 n1 + g0 + l]; rows
-    // n1 < nv of column c hold data (N2 n1 + c < lim), the rest are zeros
-    // (columns past N2, the zero-padded half of a chirped column) written
-    // directly: this buffer's previous task finished before the barrier
-    const uint32_t lg = d.lgc, G = 1u << lg, P = G + 1;
-    const uint32_t l = tid & (G - 1), S = kLongThreads >> lg;
-    const uint32_t N2 = d.N2, Nx = d.N1;
-    const uint32_t c = g0 + l;
-    const c32* src = (kind == LP_BCOL3) ? p.scratch + ln.scratch : p.in + ln.base;
-    const uint32_t lim = (kind == LP_BCOL1) ? d.N : d.M;  // chirped pass: zero beyond the line
-    const uint32_t nv = c < N2 ? min(Nx, (lim - c + N2 - 1) / N2) : 0u;
-    uint32_t i = tid >> lg;
-    c32* dp = X + i * P + l;
-    const c32* sp = src + ((uint64_t)N2 * i + c);
-    const uint64_t sstep = (uint64_t)S * N2;
-#pragma unroll 4
-    for (; i < nv; i += S) {
-      cp_async8(dp, sp);
-      sp += sstep;
-      dp += S * P;
+  };
+  if constexpr (PH == 1) {
+    const Ip<float, true, IpRows> ip{d.c, sm, p.tw, tid, kLongThreads, min(d.c.G, d.N2 - g0)};
+    if (d.blue) {
+      const c32* Tc = T + d.tn + (1u << d.tsplit);
+      const LongChirp ch{{Tc, Tc + d.cn, d.csplit}, d.N, d.minv, d.mshift};
+      ip.first(LongChirpLoad{p.in + ln.base, ch, d.N2, g0, inv});
+    } else {
+      ip.first(LongColLoad{p.in + ln.base + g0, d.N2, inv});
     }
-    for (; i < Nx; i += S) {
-      *dp = czero<float>();
-      dp += S * P;
+    landed();
+    ip.forward_mids();
+    ip.last(LongColStore{p.scratch + ln.scratch + g0, tw, d.N2, g0});
+  } else if constexpr (PH == 2) {
+    const Ip<float, false, IpRows> ip{d.r, sm, p.tw, tid, kLongThreads, min(d.r.G, d.N1 - g0)};
+    c32* rows = p.scratch + ln.scratch + (uint64_t)g0 * d.N2;
+    ip.first(IpLoad<float>{rows, (int64_t)d.N2, 1, 0});
+    landed();
+    ip.forward_mids();
+    if (d.blue) {
+      ip.centre(LongConvOp{d.bhat + (uint64_t)g0 * d.N2, d.N2});
+      ip.inverse_mids();
+      ip.final_dit(LongMidStore{rows, tw, d.N2, g0});
+    } else {
+      ip.last(LongRowStore{p.out + ln.obase + g0, d.N1, d.scale, inv ? -d.scale : d.scale});
     }
   } else {
-    // rows g0..g0+G-1 of the scratch: kLongThreads / G threads per row
-    // (a half-warp, a warp or two), each a run of consecutive values;
-    // rows past N1 are zeros
-    const uint32_t lg = d.lgr, P = (1u << lg) + 1;
-    const uint32_t N2 = d.N2, N1 = d.N1;
-    const uint32_t tpr = kLongThreads >> lg, r = tid >> (kLongThreadsLog2 - lg), lane = tid & (tpr - 1);
-    c32* dp = X + lane * P + r;
-    if (g0 + r < N1) {
-      const c32* sp = p.scratch + ln.scratch + (uint64_t)(g0 + r) * N2 + lane;
-#pragma unroll 4
-      for (uint32_t n2 = lane; n2 < N2; n2 += tpr) {
-        cp_async8(dp, sp);
-        sp += tpr;
-        dp += tpr * P;
-      }
-    } else {
-      for (uint32_t n2 = lane; n2 < N2; n2 += tpr) {
-        *dp = czero<float>();
-        dp += tpr * P;
-      }
-    }
+    const Ip<float, true, IpRows> ip{d.c, sm, p.tw, tid, kLongThreads, min(d.c.G, d.N2 - g0)};
+    ip.first(LongColLoad{p.scratch + ln.scratch + g0, d.N2, false});
+    landed();
+    ip.forward_mids();
+    const LongChirp ch{{T, T + d.cn, d.csplit}, d.N, d.minv, d.mshift};
+    ip.last(LongChirpStore{p.out + ln.obase, ch, d.N2, g0, d.scale, inv ? -d.scale : d.scale});
   }
 }
 
-// Transforms the task whose data sits in X (W: the ping-pong partner, T:
-// its table area) and stores its results.  Ends without a barrier.
-FFT_D void long_compute(const LongParams& p, const LongLenDesc& d, const LongTask& ln, uint32_t kind,
-                        c32* X, c32* W, const c32* T, uint32_t tid) {
-  const uint32_t g0 = ln.g0;
-  const bool inv = p.inverse != 0;
-  const bool colk = kind == LP_COL || kind == LP_BCOL1 || kind == LP_BCOL3;
-  const uint32_t lg = colk ? d.lgc : d.lgr, G = 1u << lg, P = G + 1;
-  const uint32_t l = tid & (G - 1), S = kLongThreads >> lg, i0 = tid >> lg;
-  const uint32_t N1 = d.N1, N2 = d.N2;
-  // input conjugation (inverse transforms) and the chirp of the first
-  // Bluestein pass, in place
-  if (kind == LP_BCOL1) {
-    const uint32_t c = g0 + l;
-    if (c < N2) {
-      uint32_t n = N2 * i0 + c;
-      ChirpWalk cw;
-      cw.init(n, S * N2, d.N, p.tw + d.ca, p.tw + d.cb, d.csplit);
-      c32* dp = X + i0 * P + l;
-      const uint32_t dn = S * N2;
-      uint32_t i = i0;
-      // four chirp values' loads in flight together
-      constexpr int U = 4;
-      for (; i + (U - 1) * S < N1 && n + (U - 1) * dn < d.N; i += U * S) {
-        c32 w[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          w[u] = cw.value_ldg();
-          cw.step();
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          c32 v = dp[u * S * P];
-          if (inv) v.im = -v.im;
-          dp[u * S * P] = cmul(v, w[u]);
-        }
-        n += U * dn;
-        dp += U * S * P;
-      }
-      for (; i < N1 && n < d.N; i += S) {
-        c32 v = *dp;
-        if (inv) v.im = -v.im;
-        *dp = cmul(v, cw.value_ldg());
-        cw.step();
-        n += dn;
-        dp += S * P;
-      }
-    }
-    __syncthreads();
-  } else if (kind == LP_COL && inv) {
-    for (uint32_t e = tid; e < N1 * P; e += kLongThreads) X[e].im = -X[e].im;
-    __syncthreads();
-  }
-  const LongSched& sch = colk ? d.s1 : d.s2;
-  if (kind == LP_COL || kind == LP_BCOL1) {
-    // scratch[k1][g0 + l] = X[k1] * W_M^{(g0+l) k1}, from the last stage
-    EpiCol e;
-    e.c = g0 + l;
-    e.ok = e.c < N2;
-    e.dst = p.scratch + ln.scratch + (e.ok ? e.c : 0);
-    e.sh = d.tsplit;
-    e.T = T;
-    e.N2 = N2;
-    ilv_fft(X, W, sch, lg, tid, T, e);
-    return;
-  }
-  if (kind == LP_ROW) {
-    // out[k1 + N1 k2], k1 = g0 + l, from the last stage
-    EpiRow e;
-    e.ok = g0 + l < N1;
-    e.dst = p.out + ln.obase + (e.ok ? g0 + l : 0);
-    e.N1 = N1;
-    e.sc = d.scale;
-    e.sci = inv ? -d.scale : d.scale;
-    ilv_fft(X, W, sch, lg, tid, T, e);
-    return;
-  }
-  c32* r = X;
-  c32* o = W;
-  // the Bluestein middle pass multiplies by the chirp spectrum at
-  // k = k1 + N1 k2 (k1 = g0 + l, k2 = i0 + m S): its values are loaded into
-  // registers now, so the loads overlap the first FFT (m < ceil(N2 / S) <= 13
-  // for the row-task shapes: G = 16 up to 208 points, 8 up to 393, 4 up to 512)
-  constexpr int kBh = 13;
-  c32 bhv[kBh];
-  const uint32_t k1m = g0 + l;
-  if (kind == LP_BMID) {
-    const c32* bh = d.bhat + (k1m < N1 ? k1m : 0) + (uint64_t)N1 * i0;
-#pragma unroll
-    for (int m = 0; m < kBh; ++m)
-      bhv[m] = (i0 + m * S < N2) ? bh[(uint64_t)m * S * N1] : czero<float>();
-  }
-  // one FFT; the Bluestein middle pass runs two with the conjugated spectrum
-  // product between them: the forward row FFT of the conjugate is the
-  // inverse row FFT
-  const int nfft = kind == LP_BMID ? 2 : 1;
-#pragma unroll 1
-  for (int f = 0; f < nfft; ++f) {
-    c32* res = ilv_fft(r, o, sch, lg, tid, T, EpiNone());
-    o = (res == r) ? o : r;
-    r = res;
-    if (f + 1 == nfft) break;
-    if (k1m < N1) {
-      c32* dp = r + i0 * P + l;
-#pragma unroll
-      for (int m = 0; m < kBh; ++m) {
-        if (i0 + m * S < N2) {
-          c32 v = cmul(dp[m * S * P], bhv[m]);
-          v.im = -v.im;
-          dp[m * S * P] = v;
-        }
-      }
-    }
-    __syncthreads();
-  }
-  // stores
-  if (kind == LP_BMID) {
-    // scratch row k1 = g0 + rr, position n2: V * W_M^{n2 k1}
-    // (kLongThreads / G threads per row, each a run of consecutive values)
-    const uint32_t tpr = kLongThreads >> lg, rr = tid >> (kLongThreadsLog2 - lg), lane = tid & (tpr - 1);
-    const uint32_t k1 = g0 + rr;
-    if (k1 < N1) {
-      c32* row = p.scratch + ln.scratch + (uint64_t)k1 * N2;
-      const c32* sp = r + lane * P + rr;
-#pragma unroll 4
-      for (uint32_t n2 = lane; n2 < N2; n2 += tpr) {
-        row[n2] = cmul(*sp, tw_two(T, kTabTa, kTabTb, n2 * k1, d.tsplit));
-        sp += tpr * P;
-      }
-    }
-  } else {  // LP_BCOL3: out[n] = conj(Y[n]) * chirp(n), n = N2 n1 + g0 + l < N
-    const uint32_t c = g0 + l;
-    if (c < N2) {
-      const float sc = d.scale;
-      uint32_t n = N2 * i0 + c;
-      ChirpWalk cw;
-      cw.init(n, S * N2, d.N, T + kTabTa, T + kTabTb, d.csplit);
-      c32* dst = p.out + ln.obase + n;
-      const c32* sp = r + i0 * P + l;
-      for (uint32_t n1 = i0; n1 < N1 && n < d.N; n1 += S) {
-        c32 wv = *sp;
-        wv.im = -wv.im;
-        c32 v = cmul(wv, cw.value());
-        v.re *= sc;
-        v.im = inv ? -v.im * sc : v.im * sc;
-        *dst = v;
-        cw.step();
-        n += S * N2;
-        dst += (uint64_t)S * N2;
-        sp += S * P;
-      }
-    }
-  }
-}
-
-// Persistent kernel of one long-line phase.  CTAs take chunks of
-// kLongChunk consecutive tasks from a work queue (one atomicAdd per
-// chunk), claimed a chunk ahead: the claim for the CTA's chunk c + 1 is
+// Persistent kernel of one long-line phase PH (= p.phase).  CTAs take
+// chunks of kLongChunk consecutive tasks from a work queue (one atomicAdd
+// per chunk), claimed a chunk ahead: the claim for the CTA's chunk c + 1 is
 // issued when it starts using chunk c and its result is stored after that
-// iteration's transform, so the atomic's latency is hidden too.  While
-// iteration k transforms the CTA's task k, asynchronous copies run three
-// stages ahead: the data and tables of task k + 1 (into the other landing
-// buffer), the length descriptor of task k + 2 (a ring of three) and the
-// record of task k + 3 (a ring of four), committed as one group and
-// waited for at the top of iteration k + 1, so no descriptor load sits on
-// the critical path.
-// One instantiation per phase PH (= p.phase), so each holds only the code
-// of its two task kinds.  Dynamic shared memory: two landing buffers and
-// one work buffer of p.cap complex values, then the two table areas of
-// kLongTab values (one per landing buffer).
+// iteration's task, so the atomic's latency is hidden too.  While iteration
+// k runs task k, asynchronous copies bring the length descriptor of task
+// k + 2 (a ring of three) and the record of task k + 3 (a ring of four).
+// Dynamic shared memory: p.cap values of data, then the tables.
 template <uint32_t PH>
-__global__ void __launch_bounds__(kLongThreads, 2) k_long_pass(const __grid_constant__ LongParams p) {
+__global__ void __launch_bounds__(kLongThreads, 4) k_long_pass(const __grid_constant__ LongParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ LongLenDesc s_len[3];
   __shared__ LongTask s_task[4];
   __shared__ uint32_t s_chunk[4];  // first task of the CTA's chunk c, at c % 4
   static_assert(sizeof(LongLenDesc) % 8 == 0, "descriptors are copied as 8-byte words");
-  c32* const base = reinterpret_cast<c32*>(smem_raw);
-  c32* const work = base + 2 * p.cap;
-  c32* const tab = base + 3 * p.cap;
+  c32* const data = reinterpret_cast<c32*>(smem_raw);
+  c32* const tab = data + p.cap;
   const uint32_t tid = threadIdx.x;
   constexpr uint32_t kNone = 0xFFFFFFFFu;
   // the CTA's k-th task (its chunk claimed and visible); kNone from the
@@ -574,7 +361,7 @@ __global__ void __launch_bounds__(kLongThreads, 2) k_long_pass(const __grid_cons
     s_chunk[1] = atomicAdd(p.counter, 1u) * kLongChunk;
   }
   __syncthreads();
-  uint32_t held0 = kNone, held1 = kNone;        // length whose tables landing buffer 0/1 holds
+  uint32_t held = kNone;  // length whose tables are in `tab`
   uint32_t ring0 = kNone, ring1 = kNone, ring2 = kNone;  // length each descriptor slot holds
   // record of task k into s_task[k % 4]
   auto fetch_task = [&](uint32_t k) {
@@ -598,19 +385,6 @@ __global__ void __launch_bounds__(kLongThreads, 2) k_long_pass(const __grid_cons
     for (uint32_t i = tid; i < sizeof(LongLenDesc) / 8; i += kLongThreads)
       cp_async8(dst + i, src + i);
   };
-  // data of task k (whose record and descriptor have landed) into landing
-  // buffer k % 2, with its length's tables when that buffer's differ
-  auto fetch_data = [&](uint32_t k) {
-    if (task_of(k) == kNone) return;
-    const LongTask& tk = s_task[k & 3];
-    const LongLenDesc& d = s_len[k % 3];
-    const uint32_t slot = k & 1;
-    const bool tables = tk.len != (slot ? held1 : held0);
-    if (slot) held1 = tk.len;
-    else held0 = tk.len;
-    long_issue(p, d, tk, long_kind(PH, d.blue != 0), base + slot * p.cap, tab + slot * kLongTab,
-               tables, tid);
-  };
   fetch_task(0);
   fetch_task(1);
   fetch_task(2);
@@ -620,26 +394,26 @@ __global__ void __launch_bounds__(kLongThreads, 2) k_long_pass(const __grid_cons
   fetch_len(0);
   fetch_len(1);
   cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();
-  fetch_data(0);
-  cp_async_commit();
 #pragma unroll 1
   for (uint32_t k = 0; task_of(k) != kNone; ++k) {
     cp_async_wait<0>();
-    __syncthreads();  // task k's data, k + 1's descriptor and k + 2's record have landed,
-                      // and every thread is past task k - 1
+    __syncthreads();  // task k's and k + 1's descriptors and k + 2's record have landed, and
+                      // every thread is past task k - 1
     // task k + 3 opens chunk c = (k + 3) / kLongChunk: claim chunk c + 1
     const bool claim = tid == 0 && (k + 3) % kLongChunk == 0;
     const uint32_t claimed = claim ? atomicAdd(p.counter, 1u) * kLongChunk : 0u;
-    fetch_data(k + 1);
+    const LongLenDesc& d = s_len[k % 3];
+    const LongTask& ln = s_task[k & 3];
+    const bool fresh = ln.len != held;
+    if (fresh) {
+      held = ln.len;
+      long_tables<PH>(p, d, tab);
+      cp_async_commit();
+    }
     fetch_len(k + 2);
     fetch_task(k + 3);
     cp_async_commit();
-    const LongLenDesc& d = s_len[k % 3];
-    const uint32_t slot = k & 1;
-    long_compute(p, d, s_task[k & 3], long_kind(PH, d.blue != 0), base + slot * p.cap, work,
-                 tab + slot * kLongTab, tid);
+    long_task<PH>(p, d, ln, data, tab, fresh);
     // first read at iteration k + 4, after the barriers between
     if (claim) s_chunk[((k + 3) / kLongChunk + 1) & 3] = claimed;
   }
