@@ -417,18 +417,32 @@ Buffer = Union["torch.Tensor", Tuple[int, int]]  # noqa: F821
 def _buf(b) -> Tuple[int, int]:
     if isinstance(b, tuple):
         return int(b[0]), int(b[1])
-    if hasattr(b, "data_ptr"):
+    try:
         if not b.is_cuda:
             raise FftError("InvalidArgument", 15, "buffers must be CUDA device memory")
-        return int(b.data_ptr()), int(b.numel() * b.element_size())
-    raise TypeError("buffer must be a torch CUDA tensor or an (address, nbytes) pair")
+        return b.data_ptr(), b.numel() * b.element_size()
+    except AttributeError:
+        raise TypeError("buffer must be a torch CUDA tensor or an (address, nbytes) pair") from None
+
+
+_current_stream = None  # the current device's current stream, as an address
 
 
 def _stream(s) -> int:
     if s is None:
+        global _current_stream
+        if _current_stream is None:
+            try:
+                import torch
+            except ImportError:
+                return 0
+            raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+            if raw is not None:  # no Stream object on each call (3 us)
+                _current_stream = lambda: raw(torch.cuda.current_device())  # noqa: E731
+            else:
+                _current_stream = lambda: int(torch.cuda.current_stream().cuda_stream)  # noqa: E731
         try:
-            import torch
-            return int(torch.cuda.current_stream().cuda_stream)
+            return _current_stream()
         except Exception:
             return 0
     if isinstance(s, int):

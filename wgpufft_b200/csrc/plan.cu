@@ -1812,71 +1812,71 @@ static b2f_status run_passes(const Plan& plan, cudaStream_t st, const void* in, 
   // earlier call of this thread left there
   cudaGetLastError();
   cudaError_t e = cudaSuccess;
-  for (const Pass& p0 : plan.passes) {
-    Pass p = p0;  // launch parameters take the caller's pointers
+  // a pass's launch parameters are copied to take the caller's pointers (the
+  // one parameter block, not the pass with its labels)
+  auto with = [](auto prm, const void* src, void* dst) {
+    prm.in = src;
+    prm.out = dst;
+    return prm;
+  };
+  for (const Pass& p : plan.passes) {
     void* src = bufs[p.src];
     void* dst = bufs[p.dst];
     switch (p.kind) {
       case Pass::LINES:
-        p.lines.in = src;
-        p.lines.out = dst;
-        e = launch_lines(plan.prec, p.lines, p.grid, p.threads, p.smem, st);
+        e = launch_lines(plan.prec, with(p.lines, src, dst), p.grid, p.threads, p.smem, st);
         break;
       case Pass::POW2: {
-        p.lines.in = src;
-        p.lines.out = dst;
+        const LinesParams lp = with(p.lines, src, dst);
         bool done = false;
         if (p.tma) {
-          const uint64_t outer = p.grid / ((uint64_t)p.lines.io.tiles * p.lines.io.mid_n);
-          done = launch_pow2_tma(p.lines, p.grid, outer, p.threads, p.tma_grid,
+          const uint64_t outer = p.grid / ((uint64_t)lp.io.tiles * lp.io.mid_n);
+          done = launch_pow2_tma(lp, p.grid, outer, p.threads, p.tma_grid,
                                  (unsigned int*)plan.device_allocs[p.tma_err], st, &e);
         }
-        if (!done) e = launch_pow2(plan.prec, p.pow2_E, p.colmajor, p.lines, p.grid, p.threads, p.smem, st);
+        if (!done) e = launch_pow2(plan.prec, p.pow2_E, p.colmajor, lp, p.grid, p.threads, p.smem, st);
         break;
       }
-      case Pass::RADER:
-        p.rader.L.in = src;
-        p.rader.L.out = dst;
-        e = launch_rader(plan.prec, p.rader, p.grid, p.threads, p.smem, st);
+      case Pass::RADER: {
+        RaderParams rp = p.rader;
+        rp.L.in = src;
+        rp.L.out = dst;
+        e = launch_rader(plan.prec, rp, p.grid, p.threads, p.smem, st);
         break;
-      case Pass::BLUESTEIN:
-        p.blue.L.in = src;
-        p.blue.L.out = dst;
-        e = launch_bluestein(plan.prec, p.blue, p.grid, p.threads, p.smem, st);
+      }
+      case Pass::BLUESTEIN: {
+        BluesteinParams bl = p.blue;
+        bl.L.in = src;
+        bl.L.out = dst;
+        e = launch_bluestein(plan.prec, bl, p.grid, p.threads, p.smem, st);
         break;
+      }
       case Pass::R2C:
-      case Pass::C2R:
-        p.real.in = src;
-        p.real.out = dst;
+      case Pass::C2R: {
+        const RealParams rp = with(p.real, src, dst);
         if (p.real_fx)
-          e = launch_real_fixed(plan.prec, p.kind == Pass::R2C, p.real, p.grid, p.threads, p.smem, st);
+          e = launch_real_fixed(plan.prec, p.kind == Pass::R2C, rp, p.grid, p.threads, p.smem, st);
         else if (p.kind == Pass::R2C)
-          e = launch_r2c(plan.prec, p.real, p.grid, p.threads, p.smem, st);
+          e = launch_r2c(plan.prec, rp, p.grid, p.threads, p.smem, st);
         else
-          e = launch_c2r(plan.prec, p.real, p.grid, p.threads, p.smem, st);
+          e = launch_c2r(plan.prec, rp, p.grid, p.threads, p.smem, st);
         break;
+      }
       case Pass::IP:
-        p.ip.in = src;
-        p.ip.out = dst;
-        e = launch_ip(plan.prec, p.ip_kind, p.ip_col, p.ip, p.grid, p.threads, p.smem, st);
+        e = launch_ip(plan.prec, p.ip_kind, p.ip_col, with(p.ip, src, dst), p.grid, p.threads,
+                      p.smem, st);
         break;
       case Pass::SCALE_COPY:
         e = launch_scale_copy(plan.prec, src, dst, p.copy_n, p.copy_scale, p.copy_conj, st);
         break;
       case Pass::BLUE_ELEM:
-        p.belem.in = src;
-        p.belem.out = dst;
-        e = launch_blue_elem(plan.prec, p.belem, st);
+        e = launch_blue_elem(plan.prec, with(p.belem, src, dst), st);
         break;
       case Pass::REAL_ELEM:
-        p.relem.in = src;
-        p.relem.out = dst;
-        e = launch_real_elem(plan.prec, p.relem, st);
+        e = launch_real_elem(plan.prec, with(p.relem, src, dst), st);
         break;
       case Pass::SMALL_VOLUME:
-        p.svol.in = src;
-        p.svol.out = dst;
-        e = launch_small_volume(plan.prec, p.svol, p.threads, p.smem, st);
+        e = launch_small_volume(plan.prec, with(p.svol, src, dst), p.threads, p.smem, st);
         break;
       case Pass::TC_DFT64:
         e = launch_dft64_tc(src, dst, (const float*)plan.device_allocs[p.tc_table], p.tc_nlines,

@@ -15,6 +15,7 @@ the trailing ones.
 """
 from __future__ import annotations
 
+import math
 from typing import Dict, Optional, Sequence, Tuple
 
 import wgpufft_b200 as w
@@ -25,7 +26,7 @@ _PLANS: Dict[tuple, w.FftPlan] = {}
 
 
 def _plan(kind, shape, axes, batch, inverse, norm, prec, device):
-    key = (int(kind), tuple(shape), tuple(axes), batch, inverse, int(norm), int(prec), device)
+    key = (kind, tuple(shape), tuple(axes), batch, inverse, norm, prec, device)
     p = _PLANS.get(key)
     if p is None:
         cfg = (w.FftConfig.new_nd(list(shape)).with_axes(list(axes)).with_batch(batch)
@@ -69,6 +70,8 @@ def _c2c(x, s, dim, norm, inverse):
     if s is not None:
         x = _resize(x, dims, s)
     x = x.contiguous()
+    if x.is_conj():
+        torch.view_as_real(x)  # raises: the conjugation is not in memory
     prec = w.FftPrecision.F64 if x.dtype == torch.complex128 else w.FftPrecision.F32
     k = x.dim()
     out = torch.empty_like(x)
@@ -77,13 +80,10 @@ def _c2c(x, s, dim, norm, inverse):
         # leading dimensions its batch, and its normalisation (1 / the
         # product of the shape) is torch's
         t = len(dims)
-        shape = list(x.shape[k - t:])[::-1]
-        batch = 1
-        for d in x.shape[:k - t]:
-            batch *= int(d)
-        plan = _plan(w.FftTransformKind.C2c, shape, list(range(t)), batch, inverse, _NORM[norm],
-                     prec, x.device.index)
-        plan.execute_checked(torch.view_as_real(x), torch.view_as_real(out))
+        dims = tuple(x.shape)
+        plan = _plan(w.FftTransformKind.C2c, dims[:k - t - 1 if t < k else None:-1], range(t),
+                     math.prod(dims[:k - t]), inverse, _NORM[norm], prec, x.get_device())
+        plan.execute_checked(x, out)
         return out
     # other subsets: the crate scales by its whole shape, torch by the
     # transformed dimensions only, so the plan runs unnormalised and the
@@ -92,7 +92,7 @@ def _c2c(x, s, dim, norm, inverse):
     axes = sorted(k - 1 - d for d in dims)
     plan = _plan(w.FftTransformKind.C2c, shape, axes, 1, inverse, w.Normalization.NONE, prec,
                  x.device.index)
-    plan.execute_checked(torch.view_as_real(x), torch.view_as_real(out))
+    plan.execute_checked(x, out)
     n = 1
     for d in dims:
         n *= int(x.shape[d])
