@@ -243,9 +243,12 @@ namespace b2f {
 // shared-memory buffer of G * LD values (exchanges and the pre/post
 // processing, which pairs k with h - k).  rtw: W_N0^k for k < h, built in
 // FP64 and rounded once.
+// f32: 64 registers, four CTAs of 256 threads an SM (no spills; at 72 and
+// three CTAs 16,384 lines of 1024 points took 40.6 us R2C and 43.8 us C2R,
+// now 37.6 and 40.8).
 template <class S>
 struct FxRealBounds {
-  static constexpr int blocks = sizeof(S) == 8 ? 2 : 3;
+  static constexpr int blocks = sizeof(S) == 8 ? 2 : 4;
 };
 
 // R2C: z[n] = x[2n] + i x[2n+1], Z = FFT_h(z), then for k <= h/2:
