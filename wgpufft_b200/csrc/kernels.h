@@ -53,6 +53,12 @@ struct LinesParams {
   const void* tws_a;
   const void* tws_b;
   FastDiv d_tws;
+  // fixed-length f32 column tiles (when tws_d is set): the same two tables in
+  // FP64, hi at 0 and lo at tws_dn; tws_t, [n][c], W_M^{c n} for the columns
+  // c < G of a tile (tw_div == 1)
+  const void* tws_d;
+  const void* tws_t;
+  uint32_t tws_dn;
   double scale;
   Schedule sch;
 };

@@ -34,6 +34,17 @@ cudaError_t launch_pow2_fixed(Prec prec, int E, bool colmajor, const LinesParams
       case 13: return fx_launch<float, 16, false, 13>(prm, grid, threads, smem, st);
       default: break;
     }
+  } else if (colmajor && E == 16 && prm.tws_d != nullptr) {
+    // the four-step twiddle factored by tile
+    switch (lg) {
+      case 4: return fx_launch<float, 16, true, 4, true>(prm, grid, threads, smem, st);
+      case 5: return fx_launch<float, 16, true, 5, true>(prm, grid, threads, smem, st);
+      case 6: return fx_launch<float, 16, true, 6, true>(prm, grid, threads, smem, st);
+      case 7: return fx_launch<float, 16, true, 7, true>(prm, grid, threads, smem, st);
+      case 8: return fx_launch<float, 16, true, 8, true>(prm, grid, threads, smem, st);
+      case 9: return fx_launch<float, 16, true, 9, true>(prm, grid, threads, smem, st);
+      default: break;
+    }
   } else if (colmajor && E == 16) {
     switch (lg) {
       case 4: return fx_launch<float, 16, true, 4>(prm, grid, threads, smem, st);

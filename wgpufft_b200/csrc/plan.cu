@@ -498,7 +498,7 @@ struct Builder {
   enum Field { F_LINES_TW, F_RADER_TW, F_BLUE_TW, F_REAL_TW, F_PERM_IN, F_PERM_OUT, F_RADER_BHAT,
                F_BLUE_BHAT, F_BELEM_BHAT, F_TWS_A, F_TWS_B, F_SVOL_TW, F_BLUE_CHIRP,
                F_BELEM_CHIRP, F_REAL_RTW, F_BELEM_PIN, F_BELEM_POUT, F_BELEM_X0,
-               F_IP_TW, F_IP_PERM, F_IP_BHAT, F_IP_CHIRP, F_IP_RTW };
+               F_TWS_D, F_TWS_T, F_IP_TW, F_IP_PERM, F_IP_BHAT, F_IP_CHIRP, F_IP_RTW };
   struct Patch {
     size_t table, pass;
     Field field;
@@ -538,6 +538,8 @@ struct Builder {
         case F_BLUE_CHIRP: ps.blue.chirp = ptr; break;
         case F_BELEM_CHIRP: ps.belem.chirp = ptr; break;
         case F_REAL_RTW: ps.real.rtw = ptr; break;
+        case F_TWS_D: ps.lines.tws_d = ptr; break;
+        case F_TWS_T: ps.lines.tws_t = ptr; break;
         case F_IP_TW: ps.ip.tw = ptr; break;
         case F_IP_PERM: ps.ip.perm = (const uint32_t*)ptr; break;
         case F_IP_BHAT: ps.ip.bhat = ptr; break;
@@ -1216,6 +1218,27 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
     b.set_table(idx, Builder::F_TWS_A, b.add_table(b.pack_complex(ta)));
     b.set_table(idx, Builder::F_TWS_B, b.add_table(b.pack_complex(tb)));
     (ps.kind == Pass::IP ? ps.ip.d_tws : ps.lines.d_tws) = make_fastdiv((uint32_t)L);
+    // the fixed-length f32 column tiles factor the twiddle by tile
+    // (fx_tile_twiddles): both tables in FP64 and, where adjacent columns are
+    // adjacent rows, the tile's own table
+    LinesParams& lp = ps.lines;
+    if (ps.kind != Pass::POW2 || !ps.colmajor || ps.pow2_E != 16 || b.plan.prec != PREC_F32 ||
+        M > 0xFFFFFFFFull || ps.tma || (lp.io.tw_div == 1 && lp.N > 256))
+      return;
+    std::vector<cd> d = ta;
+    d.insert(d.end(), tb.begin(), tb.end());
+    std::vector<unsigned char> bytes(d.size() * sizeof(cd));
+    std::memcpy(bytes.data(), d.data(), bytes.size());
+    lp.tws_dn = (uint32_t)ta.size();
+    b.set_table(idx, Builder::F_TWS_D, b.add_table(std::move(bytes)));
+    if (lp.io.tw_div == 1) {
+      const RootProduct root(M);
+      std::vector<cd> t;
+      for (uint64_t n = 0; n < lp.N; ++n)
+        for (uint64_t c = 0; c < lp.G; ++c) t.push_back(root(c * n % M));
+      b.set_table(idx, Builder::F_TWS_T, b.add_table(b.pack_complex(t)));
+    }
+    ps.smem += (size_t)lp.N * b.cb();
   };
   {
     // pass A: columns n1 (stride N2*s), W_N^{n2 k1} on store, src -> ws

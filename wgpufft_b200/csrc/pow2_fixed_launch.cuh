@@ -5,10 +5,10 @@
 
 namespace b2f {
 
-template <class S, int E, bool COLMAJOR, int LOGN>
+template <class S, int E, bool COLMAJOR, int LOGN, bool TT = false>
 inline cudaError_t fx_launch(const LinesParams& prm, unsigned grid, unsigned threads, size_t smem,
                              cudaStream_t st) {
-  return launch(k_pow2_fx<S, E, COLMAJOR, LOGN>, prm, grid, threads, smem, st);
+  return launch(k_pow2_fx<S, E, COLMAJOR, LOGN, TT>, prm, grid, threads, smem, st);
 }
 
 // f64 and df64 (16 values a thread, lines of up to 4096 points)

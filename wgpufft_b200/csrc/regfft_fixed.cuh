@@ -112,6 +112,30 @@ FFT_D void fx_stages(cpx<S> (&v)[E], cpx<S>* line, uint32_t t, const cpx<S>* __r
   }
 }
 
+// The twiddle on store of a column tile, W_M^{row(c) n} = T1[n] * T2[n][c]:
+// T1[n] = W_M^{row0 n}, row0 the tile's first row, is computed once a tile
+// in FP64 (one value a thread) and rounded to a shared-memory table of N
+// values; T2 = W_M^{(row(c) - row0) n} is 1 when the tile has one row and
+// otherwise a table shared by every tile, read with adjacent columns side by
+// side.  Looking W_M^{row n} up in the two sqrt(M) tables for every value
+// scatters each load over up to 32 cache lines: one line of 2^24 points
+// 212 -> 201 us, 4096 x 2048 100 -> 93 us, 256 x 65536 132 -> 126 us.
+// Tiles of 512-point columns (8 adjacent rows) are faster with the two
+// tables (64 x 2^18 161 against 167 us), so the planner builds T2 for up to
+// 256 points; kernels of their own (TT), as the code costs passes without a
+// twiddle 3 %.
+template <int N>
+FFT_D void fx_tile_twiddles(const LinesParams& p, c32* t1, uint32_t row0, uint32_t tid, uint32_t T) {
+  const double2* __restrict__ hi = (const double2*)p.tws_d;
+  const double2* __restrict__ lo = hi + p.tws_dn;
+  const uint32_t sh = p.d_tws.shift, msk = (1u << sh) - 1;
+  for (uint32_t n = tid; n < (uint32_t)N; n += T) {
+    const uint32_t m = row0 * n;  // < M <= 2^32 - 1
+    const double2 a = hi[m >> sh], b = lo[m & msk];
+    t1[n] = c32{(float)(a.x * b.x - a.y * b.y), (float)(a.x * b.y + a.y * b.x)};
+  }
+}
+
 // G lines of N = 2^LOGN points; blockDim = G * N / E (256 for 16-value
 // column tiles, up to 512 otherwise).  Shared memory: G * LD values,
 // LD = N + N/16 + 1.  f32 register budgets: 64 for contiguous lines (4
@@ -123,7 +147,7 @@ struct FxBounds {
   static constexpr int threads = wide || (COLMAJOR && E == 16) ? 256 : 512;
   static constexpr int blocks = wide ? 2 : (COLMAJOR ? (E == 16 ? 3 : 1) : 2);
 };
-template <class S, int E, bool COLMAJOR, int LOGN>
+template <class S, int E, bool COLMAJOR, int LOGN, bool TT = false>
 __global__ void __launch_bounds__(FxBounds<S, E, COLMAJOR>::threads, FxBounds<S, E, COLMAJOR>::blocks)
     k_pow2_fx(const __grid_constant__ LinesParams p) {
   using P = P2Sched<LOGN>;
@@ -166,9 +190,52 @@ __global__ void __launch_bounds__(FxBounds<S, E, COLMAJOR>::threads, FxBounds<S,
     for (int i = 0; i < E; ++i) v[i] = czero<S>();
   }
   C* line = sm + c * LD;
+  // TT: the tile's twiddles, while the first loads are in flight
+  bool tile_tw = false, one_row = false;
+  C* t1 = sm + G * LD;
+  if constexpr (TT) {
+    const uint32_t row0 = fdiv((uint32_t)g.c0, p.d_tw);
+    one_row = fdiv((uint32_t)g.c0 + g.nvalid - 1, p.d_tw) == row0;
+    tile_tw = one_row || p.tws_t != nullptr;
+    if (tile_tw) {
+      fx_tile_twiddles<N>(p, t1, row0, tid, blockDim.x);
+      if (P::NST == 1) __syncthreads();
+    }
+  }
   fx_stages<S, LOGN, 0, E>(v, line, t, tw);
   const S sc = Scalar<S>::from_double(p.scale);
   const uint32_t fl = p.flags;
+  if constexpr (TT) {
+    if (tile_tw) {
+      if (!valid) return;
+      const C* __restrict__ t2 = (const C*)p.tws_t + c;
+      C* __restrict__ dst = (C*)p.out + g.out0 + (int64_t)c * g.dl_out;
+      const int64_t es = p.io.out_es;
+#pragma unroll
+      for (int u = 0; u < E / RL; ++u) {
+        const uint32_t j = t + u * TL;
+        C* b = dst + (int64_t)j * es;
+        C w[RL];
+        if (!one_row) {
+#pragma unroll
+          for (int r = 0; r < RL; ++r) w[r] = t2[(j + r * NSL) * G];
+#pragma unroll
+          for (int r = 0; r < RL; ++r) w[r] = cmul(w[r], t1[j + r * NSL]);
+        } else {
+#pragma unroll
+          for (int r = 0; r < RL; ++r) w[r] = t1[j + r * NSL];
+        }
+#pragma unroll
+        for (int r = 0; r < RL; ++r) {
+          C x = cmul(v[u * RL + r], w[r]);
+          if (fl & PF_SCALE) x = cscale(x, sc);
+          if (fl & PF_CONJ_OUT) x.im = -x.im;
+          b[(int64_t)r * NSL * es] = x;
+        }
+      }
+      return;
+    }
+  }
   if (!(fl & PF_STORE_SMEM)) {
     // last stage: output n = j + r*NSL (j < NSL) straight to HBM
     if (!valid) return;
