@@ -95,9 +95,6 @@ FFT_D void cp_async8(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-FFT_D void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
 
 template <class T>
 FFT_D void copy_words(T* dst, const T* src, uint32_t tid, uint32_t nthreads) {

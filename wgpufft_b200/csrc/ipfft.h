@@ -71,7 +71,8 @@ bool ip_schedule(uint64_t n, bool row, bool conv, int pair, IpSched& sc,
                  std::vector<uint32_t>& radices, std::vector<std::complex<double>>& tw);
 // Frequency held by value pos of sub-line k0.
 uint32_t ip_frequency(const IpSched& sc, uint32_t k0, uint32_t pos);
-// Values of shared memory a line takes (rows).
+// Values between the sub-lines of a row: odd, so that adjacent sub-lines fall
+// into different banks.
 inline uint32_t ip_pitch(uint32_t ns) { return ns | 1u; }
 
 cudaError_t launch_ip(Prec p, IpKind kind, bool col, const IpParams& prm, unsigned grid,
