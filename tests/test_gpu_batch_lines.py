@@ -48,3 +48,43 @@ def test_a_line_alone_equals_the_same_line_among_others():
     out = torch.empty_like(d)
     w.FftBatch(lengths, off).execute(d, out)
     assert torch.equal(out[off[1]:off[1] + n], alone)
+
+
+@pytest.mark.parametrize("n", [5003, 6000, 15015, 65521])
+@pytest.mark.parametrize("count", [1, 7, 40])
+def test_few_long_lines_take_one_task_a_cta(n, count):
+    """As long as a phase has fewer tasks than CTAs fit (two an SM at least),
+    every task has a CTA of its own."""
+    lengths = np.full(count, n)
+    off = workloads.packed_offsets(lengths)
+    x = workloads.normal_complex(int(lengths.sum()), n)
+    d = torch.from_numpy(x).cuda()
+    out = torch.empty_like(d)
+    b = w.FftBatch(lengths, off)
+    b.execute(d, out)
+    ref = np.fft.fft(x.reshape(count, n).astype(np.complex128))
+    y = out.cpu().numpy().reshape(count, n)
+    assert np.all(np.linalg.norm(y - ref, axis=1) <= 2e-6 * np.linalg.norm(ref, axis=1))
+    info = b.diagnostics()
+    most = max(info["long_tasks"])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert info["long_grid"] >= min(most, 2 * sms)
+
+
+def test_tasks_dealt_out_and_from_the_queue_agree():
+    """Either side of the count from which tasks come from the work queue:
+    the same lines, bit for bit (a line's arithmetic depends on neither)."""
+    n = 6000
+    few, many = 9000, 10000
+    g = torch.Generator(device="cuda").manual_seed(5)
+    d = torch.randn(many * n, dtype=torch.complex64, device="cuda", generator=g)
+    grids, outs = [], []
+    for count in (few, many):
+        b = w.FftBatch(np.full(count, n), np.arange(count) * n)
+        info = b.diagnostics()
+        grids.append(info["long_tasks"][0] / info["long_grid"])
+        out = torch.empty_like(d[:count * n])
+        b.execute(d[:count * n], out)
+        outs.append(out)
+    assert grids[0] <= 32 < grids[1], grids
+    assert torch.equal(outs[0], outs[1][:few * n])

@@ -146,7 +146,7 @@ struct BatchPlan {
   cudaEvent_t hev_in[kHostChunks] = {}, hev_c[kHostChunks] = {};
   uint32_t long_cap = 0, long_tab = 0;  // values of data and of tables a task needs
   size_t smem_long = 0;
-  unsigned grid_long = 0;
+  unsigned grid_long = 0, resident_long = 0;  // CTAs of the largest phase; CTAs that fit
   uint64_t lines_long = 0, elems_long = 0;
   unsigned grid_big = 0;
   uint32_t buf_cta = 0, buf_cl = 0;
@@ -591,6 +591,28 @@ static cudaError_t set_smem(K kernel, size_t smem) {
                               std::max<int>(room, (int)smem));
 }
 
+// CTAs of a long phase: tasks that are dealt out have one each as far as they
+// fit, tasks of the queue one a chunk.
+static bool long_spread(uint64_t tasks, unsigned resident) {
+  return tasks <= (uint64_t)kLongSpread * resident;
+}
+static unsigned long_grid(uint64_t tasks, unsigned resident) {
+  return (unsigned)std::min<uint64_t>(
+      resident, long_spread(tasks, resident) ? tasks : (tasks + kLongChunk - 1) / kLongChunk);
+}
+
+// Launches phase ph (0..2) over lp.ntasks tasks.
+static cudaError_t launch_long_phase(LongParams& lp, uint32_t ph, unsigned resident, size_t smem,
+                                     cudaStream_t st) {
+  lp.phase = ph + 1;
+  lp.spread = long_spread(lp.ntasks, resident);
+  const unsigned grid = long_grid(lp.ntasks, resident);
+  if (ph == 0) k_long_pass<1><<<grid, kLongThreads, smem, st>>>(lp);
+  else if (ph == 1) k_long_pass<2><<<grid, kLongThreads, smem, st>>>(lp);
+  else k_long_pass<3><<<grid, kLongThreads, smem, st>>>(lp);
+  return cudaGetLastError();
+}
+
 static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets, uint64_t nlines,
                                int32_t direction, int32_t normalization, int device,
                                uint32_t flags, BatchPlan** out) {
@@ -657,20 +679,26 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
                   "UnsupportedLength { len: " + std::to_string(lens_list[i]) + " } in a batch");
     }
   bp->distinct = lens_list.size();
-  // A batch with few long lines takes smaller tasks, so that a phase has
-  // three tasks for each of the CTAs that fit (four an SM): 100 lines of
-  // 1,400 to 2,300 points as one task a line and phase took 132 us against
-  // 91 with several.  (The values a task holds do not change a line's
-  // arithmetic.)
-  for (uint64_t values = kLongTaskValues; values >= 512; values /= 2) {
-    uint64_t tasks = 0;
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+  // A batch with few long lines takes smaller tasks, down to about 1,000
+  // values (four a thread), until a phase has two tasks an SM, half of what
+  // is resident: 64 lines of 10,007 points 41 -> 33 us, 16 of 65,521 56 -> 48.
+  // Halving them until every resident CTA has two instead leaves batches of a
+  // few hundred lines with twice the stage rounds (64 x 10,007 55 us, 370
+  // lines of up to 15,000 points 54 against 40).  (The values a task holds do
+  // not change a line's arithmetic.)
+  for (uint64_t values = kLongTaskValues; values >= 1000; values /= 2) {
+    uint64_t columns = 0, rows = 0;
     for (size_t i = 0; i < infos.size(); ++i) {
       if (infos[i].d.kind != BK_LONG && infos[i].d.kind != BK_LONG_BLUE) continue;
       LongLenDesc& g = infos[i].lng;
       set_long_tasks(g, values);
-      tasks += by_len[lens_list[i]].size() * ((g.N2 + g.c.G - 1) / g.c.G);
+      const uint64_t n = by_len[lens_list[i]].size();
+      columns += n * ((g.N2 + g.c.G - 1) / g.c.G);
+      rows += n * ((g.N1 + g.r.G - 1) / g.r.G);
     }
-    if (tasks >= 3 * 4 * 148) break;
+    if (std::min(columns, rows) >= 2ull * nsm) break;
   }
   // twiddle tables shared by every length of the batch
   {
@@ -1031,8 +1059,6 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
     cudaMemcpy(bp->d_long_tasks_chunked, ltc.data(), ltc.size() * sizeof(LongTask), cudaMemcpyHostToDevice);
   }
   // launch shapes
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   if (bp->n_cta) {
     if (set_smem(k_batch_cta, bp->smem_cta) != cudaSuccess)
       return fail(B2F_ERR_DEVICE, "batch CTA kernel shared memory");
@@ -1050,9 +1076,8 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_long_pass<2>, kLongThreads, bp->smem_long);
     per_sm = std::max(per_sm, 1);
-    uint32_t most = std::max(bp->long_count[0], std::max(bp->long_count[1], bp->long_count[2]));
-    bp->grid_long = (unsigned)std::min<uint64_t>((uint64_t)nsm * per_sm,
-                                                 (most + kLongChunk - 1) / kLongChunk);
+    bp->resident_long = (unsigned)nsm * per_sm;
+    for (uint32_t n : bp->long_count) bp->grid_long = std::max(bp->grid_long, long_grid(n, bp->resident_long));
   }
   if (bp->n_cl) {
     if (set_smem(k_batch_cluster<kClusterP>, bp->smem_cl) != cudaSuccess)
@@ -1242,13 +1267,8 @@ static void launch_long(const BatchPlan& bp, cudaStream_t st, const void* in, vo
       if (count == 0) continue;
       lp.tasks = (chunk < 0 ? bp.d_long_tasks : bp.d_long_tasks_chunked) + bp.long_first[ph] + first;
       lp.ntasks = count;
-      lp.phase = ph + 1;
       lp.counter = bp.d_counters + (chunk < 0 ? 4 + ph : 9 + 4 * chunk + ph);
-      const unsigned grid = (unsigned)std::min<uint64_t>(bp.grid_long, (count + kLongChunk - 1) / kLongChunk);
-      if (ph == 0) k_long_pass<1><<<grid, kLongThreads, bp.smem_long, st>>>(lp);
-      else if (ph == 1) k_long_pass<2><<<grid, kLongThreads, bp.smem_long, st>>>(lp);
-      else k_long_pass<3><<<grid, kLongThreads, bp.smem_long, st>>>(lp);
-      e = cudaGetLastError();
+      e = launch_long_phase(lp, ph, bp.resident_long, bp.smem_long, st);
     }
   }
   *err = e;
@@ -1429,12 +1449,11 @@ static int64_t registry_add(LineRegistry& r, uint64_t n) {
   std::unique_ptr<LenInfo> li(new LenInfo());
   const size_t cta_cap = 44 * 1024;  // the batch kernels' four-CTA share of an SM
   // (a registered length does not know how many lines will share a launch:
-  // half-size long tasks)
+  // whole long tasks, 10 % faster than halves over 1 to 5,000 lines of 3,000
+  // to 65,536 points, and up to 30 % from 300 lines on)
   if (n >= 2 && n <= 0xFFFFFFFFull && r.infos.size() < kRegLengths &&
       classify(n, r.direction, r.normalization, cta_cap, r.cl_cap, false, *li) &&
       li->d.kind != BK_CL_MIXED && li->d.kind != BK_CL_BLUE) {
-    if (li->d.kind == BK_LONG || li->d.kind == BK_LONG_BLUE)
-      set_long_tasks(li->lng, kLongTaskValues / 2);
     std::vector<cd> tw;
     length_twiddles(*li, tw, r.tw_used);
     bool ok = r.tw_used + tw.size() <= kRegTwiddles;
@@ -1675,14 +1694,8 @@ b2f_status line_batch_run(LineRegistry* reg, cudaStream_t st, const uint64_t* le
       if (count) {
         lp.tasks = d_lt + first;
         lp.ntasks = (uint32_t)count;
-        lp.phase = ph + 1;
         lp.counter = counters + 4 + ph;
-        const unsigned grid = (unsigned)std::min<uint64_t>(
-            (uint64_t)reg->nsm * std::max(reg->long_per_sm, 1), (count + kLongChunk - 1) / kLongChunk);
-          if (ph == 0) k_long_pass<1><<<grid, kLongThreads, smem_long, st>>>(lp);
-        else if (ph == 1) k_long_pass<2><<<grid, kLongThreads, smem_long, st>>>(lp);
-        else k_long_pass<3><<<grid, kLongThreads, smem_long, st>>>(lp);
-        e = cudaGetLastError();
+        e = launch_long_phase(lp, ph, (unsigned)(reg->nsm * std::max(reg->long_per_sm, 1)), smem_long, st);
       }
       first += count;
     }

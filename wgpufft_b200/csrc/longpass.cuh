@@ -20,13 +20,16 @@
 // never leaving the digit-reversed order in between; and the inverse column
 // pass, chirped into the output.  One scratch region of M values per line.
 //
-// The work queue hands out chunks of consecutive tasks (mostly one line); a
-// task's record and length descriptor arrive by asynchronous copies two and
-// three tasks ahead, the two-level tables of its length (W_M, and the
-// chirp) when they differ from the last task's.  The data itself is not
-// prefetched: four CTAs of 256 threads and 64 registers share an SM and
-// cover each other's loads (fetching the next task's data or tables into L2
-// ahead cost its instructions and 3 % instead).
+// Up to kLongSpread tasks a resident CTA are dealt out, task k of CTA b being
+// b + k * gridDim.x: a batch with fewer tasks than CTAs has one a CTA.  More
+// come from a work queue in chunks of consecutive tasks (mostly one line),
+// which evens out what tasks of many lengths take.  A task's record and length
+// descriptor arrive by asynchronous copies two and three tasks ahead, the
+// two-level tables of its length (W_M, and the chirp) when they differ from
+// the last task's.  The data itself is not prefetched: four CTAs of 256
+// threads and 64 registers share an SM and cover each other's loads (fetching
+// the next task's data or tables into L2 ahead cost its instructions and 3 %
+// instead).
 //
 // What bounds it: instruction issue, 335 thread instructions per point of
 // the 20,000-line mixed workload (540 with the earlier ping-pong stages and
@@ -42,6 +45,15 @@ namespace b2f {
 
 constexpr uint32_t kLongThreads = 256;
 constexpr uint32_t kLongChunk = 4;  // consecutive tasks per work-queue claim
+// Tasks a resident CTA up to which they are dealt out.  A CTA holds four to
+// eight tasks of the queue from its start, so that small batches ran theirs
+// one after the other in a quarter of the CTAs: us from the queue / dealt out,
+// one line of 3,001 points 55.6 / 22.7, 300 of 6,000 67.7 / 28.7, 64 of 65,536
+// 87.3 / 45.9.  With 20 to 32 tasks a CTA dealing is still ahead (20,000 lines
+// of up to 15,000 points 783 / 752, 2,400 of 20,000 442 / 412); at 40 to 65
+// the queue is (10,000 of up to 65,536 1597 / 1631, 4,800 of 10,007 1273 /
+// 1316), at 100 neither (20,000 of up to 65,536).
+constexpr uint32_t kLongSpread = 32;
 // k_long_pass claims the first two chunks before its loop and every later
 // one when the chunk before it opens (three tasks ahead): that covers every
 // chunk only when a chunk holds at least three tasks
@@ -97,6 +109,7 @@ struct LongParams {
   uint32_t phase;    // 1: column pass, 2: row pass, 3: Bluestein inverse columns
   uint32_t inverse;
   uint32_t cap;      // complex elements of the data buffer
+  uint32_t spread;   // tasks are dealt out, not taken from the queue
   unsigned int* counter;  // work queue: chunks of kLongChunk tasks handed out in order
 };
 
@@ -331,13 +344,14 @@ FFT_D void long_task(const LongParams& p, const LongLenDesc& d, const LongTask& 
   }
 }
 
-// Persistent kernel of one long-line phase PH (= p.phase).  CTAs take
-// chunks of kLongChunk consecutive tasks from a work queue (one atomicAdd
-// per chunk), claimed a chunk ahead: the claim for the CTA's chunk c + 1 is
-// issued when it starts using chunk c and its result is stored after that
-// iteration's task, so the atomic's latency is hidden too.  While iteration
-// k runs task k, asynchronous copies bring the length descriptor of task
-// k + 2 (a ring of three) and the record of task k + 3 (a ring of four).
+// Persistent kernel of one long-line phase PH (= p.phase).  Tasks that are
+// not dealt out (p.spread) come in chunks of kLongChunk consecutive ones from
+// a work queue (one atomicAdd per chunk), claimed a chunk ahead: the claim for
+// the CTA's chunk c + 1 is issued when it starts using chunk c and its result
+// is stored after that iteration's task, so the atomic's latency is hidden
+// too.  While iteration k runs task k, asynchronous copies bring the length
+// descriptor of task k + 2 (a ring of three) and the record of task k + 3 (a
+// ring of four).
 // Dynamic shared memory: p.cap values of data, then the tables.
 template <uint32_t PH>
 __global__ void __launch_bounds__(kLongThreads, 4) k_long_pass(const __grid_constant__ LongParams p) {
@@ -350,13 +364,14 @@ __global__ void __launch_bounds__(kLongThreads, 4) k_long_pass(const __grid_cons
   c32* const tab = data + p.cap;
   const uint32_t tid = threadIdx.x;
   constexpr uint32_t kNone = 0xFFFFFFFFu;
-  // the CTA's k-th task (its chunk claimed and visible); kNone from the
-  // first one past the end (the queue hands out chunks in increasing order)
+  // the CTA's k-th task (of the queue: its chunk claimed and visible); kNone
+  // from the first one past the end (the queue hands out chunks in increasing order)
   auto task_of = [&](uint32_t k) -> uint32_t {
-    const uint64_t t = (uint64_t)s_chunk[(k / kLongChunk) & 3] + k % kLongChunk;
+    const uint64_t t = p.spread ? blockIdx.x + (uint64_t)k * gridDim.x
+                                : (uint64_t)s_chunk[(k / kLongChunk) & 3] + k % kLongChunk;
     return t < p.ntasks ? (uint32_t)t : kNone;
   };
-  if (tid == 0) {
+  if (tid == 0 && !p.spread) {
     s_chunk[0] = atomicAdd(p.counter, 1u) * kLongChunk;
     s_chunk[1] = atomicAdd(p.counter, 1u) * kLongChunk;
   }
@@ -400,7 +415,7 @@ __global__ void __launch_bounds__(kLongThreads, 4) k_long_pass(const __grid_cons
     __syncthreads();  // task k's and k + 1's descriptors and k + 2's record have landed, and
                       // every thread is past task k - 1
     // task k + 3 opens chunk c = (k + 3) / kLongChunk: claim chunk c + 1
-    const bool claim = tid == 0 && (k + 3) % kLongChunk == 0;
+    const bool claim = tid == 0 && !p.spread && (k + 3) % kLongChunk == 0;
     const uint32_t claimed = claim ? atomicAdd(p.counter, 1u) * kLongChunk : 0u;
     const LongLenDesc& d = s_len[k % 3];
     const LongTask& ln = s_task[k & 3];
