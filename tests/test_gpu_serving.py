@@ -181,6 +181,35 @@ def test_lines_of_different_lengths_share_one_launch(cuda):
         solo.close()
 
 
+@pytest.mark.parametrize("descending", [False, True])
+def test_every_short_length_joins_the_batched_launch(cuda, descending):
+    """All lengths of one CTA, registered in either order, fit the registry's
+    twiddle arena: every request joins a line group."""
+    import torch
+    lengths = list(range(17, 2802))
+    if descending:
+        lengths.reverse()
+    off = np.concatenate([[0], np.cumsum(lengths)])
+    x = (np.random.default_rng(4).standard_normal(2 * off[-1])).astype(np.float32)
+    d = torch.from_numpy(x).cuda()
+    out = torch.empty_like(d)
+    srv = w.FftServer(streams=2)
+    srv.hold()
+    for n, o in zip(lengths, off):
+        srv.submit_device(w.FftConfig.new(n), w.FftTransformKind.C2c, d[2 * o:2 * (o + n)],
+                          out[2 * o:2 * (o + n)])
+    srv.hold(False)
+    srv.drain(120.0)
+    st = srv.stats()
+    assert st["failed"] == 0 and st["coalesced_requests"] == len(lengths), st
+    assert st["groups"] == st["line_groups"], st
+    z = x.view(np.complex64).astype(np.complex128)
+    y = out.cpu().numpy().view(np.complex64)
+    for n, o in zip(lengths, off):
+        assert O.rel_l2(y[o:o + n], np.fft.fft(z[o:o + n])) <= 2e-6, n
+    srv.close()
+
+
 def test_device_buffer_requests(cuda):
     import torch
     rng = np.random.default_rng(8)

@@ -1373,6 +1373,10 @@ struct LineRegistry {
   LongLenDesc* d_long_lens = nullptr;
   c32* d_tw = nullptr;
   uint64_t tw_used = 0;
+  // stage tables in the arena by transform length: the one-CTA lengths up to
+  // 2,801, whose convolutions share 406 transform lengths, need 0.5 million
+  // values together and 8 million with tables of their own
+  LongCache stages;
   std::vector<void*> tables;
   uint64_t table_bytes = 0;
   size_t cl_cap = 0;
@@ -1391,19 +1395,18 @@ struct LineRegistry {
   }
 };
 
-// The twiddles one length reads (stage tables of its passes, the inter-pass
-// two-level table, the chirp tables), with offsets relative to `base`.
-static void length_twiddles(LenInfo& li, std::vector<cd>& tw, uint64_t base) {
+// The twiddles one length adds to those registered before it (stage tables of
+// its passes unless `stages` has them, the inter-pass two-level table, the
+// chirp tables), with offsets relative to `base`.
+static void length_twiddles(LenInfo& li, std::vector<cd>& tw, uint64_t base, LongCache& stages) {
   std::map<uint32_t, uint32_t> cache;
   BatchLen& d = li.d;
   if (d.kind == BK_LONG || d.kind == BK_LONG_BLUE) {
-    LongCache long_cache;
-    long_tables_of(li.lng, tw, base, long_cache);
+    long_tables_of(li.lng, tw, base, stages);
     return;
   }
   if (d.kind != BK_MIXED || d.N > 16) {
-    LongCache long_cache;
-    cta_tables_of(d, tw, base, long_cache);
+    cta_tables_of(d, tw, base, stages);
     return;
   }
   attach_stage_table(d.sch, tw, cache);
@@ -1455,7 +1458,7 @@ static int64_t registry_add(LineRegistry& r, uint64_t n) {
       classify(n, r.direction, r.normalization, cta_cap, r.cl_cap, false, *li) &&
       li->d.kind != BK_CL_MIXED && li->d.kind != BK_CL_BLUE) {
     std::vector<cd> tw;
-    length_twiddles(*li, tw, r.tw_used);
+    length_twiddles(*li, tw, r.tw_used, r.stages);
     bool ok = r.tw_used + tw.size() <= kRegTwiddles;
     if (ok && !tw.empty()) {
       std::vector<float> f(tw.size() * 2);
@@ -1509,7 +1512,12 @@ static int64_t registry_add(LineRegistry& r, uint64_t n) {
         idx = -1;
       }
     }
-    if (!ok) cudaGetLastError();
+    if (!ok) {
+      cudaGetLastError();
+      // the stage tables this length would have added
+      for (auto s = r.stages.begin(); s != r.stages.end();)
+        s = s->second.second >= r.tw_used ? r.stages.erase(s) : std::next(s);
+    }
   }
   r.index[n] = idx;
   return idx;
