@@ -88,3 +88,27 @@ def test_tasks_dealt_out_and_from_the_queue_agree():
         outs.append(out)
     assert grids[0] <= 32 < grids[1], grids
     assert torch.equal(outs[0], outs[1][:few * n])
+
+
+@pytest.mark.parametrize("inverse", [False, True])
+@pytest.mark.parametrize("count", [1, 3, 150, 1000, 40000])
+@pytest.mark.parametrize("n", [13, 16, 17, 32, 122, 1009, 2600])
+def test_tasks_of_short_lines(n, count, inverse):
+    """One task, a task for every CTA, and more than that (the queue); few
+    lines are spread over the chip, not packed into full tasks."""
+    if n * count > 1 << 24:
+        pytest.skip("more points than this needs")
+    b = w.FftBatch(np.full(count, n), np.arange(count) * n,
+                   direction=w.FftDirection.Inverse if inverse else w.FftDirection.Forward)
+    x = workloads.normal_complex(count * n, n)
+    d = torch.from_numpy(x).cuda()
+    out = torch.empty_like(d)
+    for _ in range(2):  # a second call finds the queue as it must be
+        out.zero_()
+        b.execute(d, out)
+    z = x.reshape(count, n).astype(np.complex128)
+    ref = np.fft.ifft(z) if inverse else np.fft.fft(z)
+    y = out.cpu().numpy().reshape(count, n)
+    assert np.all(np.linalg.norm(y - ref, axis=1) <= 2e-6 * np.linalg.norm(ref, axis=1))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert b.diagnostics()["cta_tasks"] >= min(count, 2 * sms, count * n // 1500)

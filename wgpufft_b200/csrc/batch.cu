@@ -591,6 +591,23 @@ static cudaError_t set_smem(K kernel, size_t smem) {
                               std::max<int>(room, (int)smem));
 }
 
+// What the lines of a CTA task (G of each length, filling the CTA's share of
+// the shared memory) are divided by, 1, 2 or 4, until the batch has two tasks
+// an SM: a task's loads, stages and stores follow one another, so that few
+// full tasks leave the chip idle (148 lines of 2,600 points as 74 tasks 16.4
+// us, as 148 12.3; 300 of 32 points as 3 tasks 12.3, as 11 8.2).  Dividing by
+// 8, or until there are four an SM, costs batches of many short lines more
+// than it gives (20,000 of 32 points 12.4 -> 16.2 us, 600 of 1,009 21 -> 27).
+static uint32_t cta_divisor(const std::vector<std::pair<uint32_t, uint64_t>>& lens, int nsm) {
+  uint32_t div = 1;
+  for (; div < 4; div *= 2) {
+    uint64_t tasks = 0;
+    for (const auto& [G, lines] : lens) tasks += (lines + std::max(1u, G / div) - 1) / std::max(1u, G / div);
+    if (tasks >= 2ull * nsm) break;
+  }
+  return div;
+}
+
 // CTAs of a long phase: tasks that are dealt out have one each as far as they
 // fit, tasks of the queue one a chunk.
 static bool long_spread(uint64_t tasks, unsigned resident) {
@@ -846,6 +863,10 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
   }
   // tasks: CTA tasks (groups of G lines of one length and one chunk),
   // cluster tasks (one line each)
+  std::vector<std::pair<uint32_t, uint64_t>> cta_lens;
+  for (size_t li = 0; li < lens_list.size(); ++li)
+    if (infos[li].d.kind <= BK_BLUE) cta_lens.push_back({infos[li].d.G, by_len[lens_list[li]].size()});
+  const uint32_t cta_div = cta_divisor(cta_lens, nsm);
   std::vector<uint64_t> sorted_off;
   std::vector<BatchTask> cta_tasks, cl_tasks, big_tasks, cta_ch_tasks;
   std::vector<double> cta_cost, cl_cost, big_cost, cta_ch_cost;
@@ -918,8 +939,9 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
       }
       continue;
     }
-    for (size_t s = 0; s < ls.size(); s += d.G) {
-      const BatchTask t = make(s, std::min<size_t>(ls.size(), s + d.G), 0);
+    const uint32_t G = std::max(1u, d.G / cta_div);
+    for (size_t s = 0; s < ls.size(); s += G) {
+      const BatchTask t = make(s, std::min<size_t>(ls.size(), s + G), 0);
       cta_tasks.push_back(t);
       cta_cost.push_back(infos[li].cost * t.count);
       bp->lines_cta += t.count;
@@ -928,7 +950,7 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
     for (size_t s = 0; s < ls.size();) {
       const uint32_t ch = chunk_of[ls[s]];
       size_t e = s;
-      while (e < ls.size() && chunk_of[ls[e]] == ch && e - s < d.G) ++e;
+      while (e < ls.size() && chunk_of[ls[e]] == ch && e - s < G) ++e;
       cta_ch_tasks.push_back(make(s, e, ch));
       cta_ch_cost.push_back(infos[li].cost * (double)(e - s));
       s = e;
@@ -1177,7 +1199,15 @@ static b2f_status run_batch(const BatchPlan& bp, cudaStream_t st, const void* in
   int prev = -1;
   cudaGetDevice(&prev);
   if (prev != bp.device) cudaSetDevice(bp.device);
-  cudaError_t e = cudaMemsetAsync(bp.d_counters, 0, kBatchCounters * sizeof(unsigned int), st);
+  const bool run_cl = (bp.n_cl || bp.n_big) && (parts & 2);
+  const bool run_cta = bp.n_cta && (parts & 1);
+  const bool run_long = bp.lines_long && (parts & 4);
+  // launches with a CTA for every task, or whose tasks are dealt out, leave
+  // the counters alone
+  bool queues = run_cl || (run_cta && bp.grid_cta < bp.n_cta);
+  for (uint32_t n : bp.long_count) queues = queues || (run_long && !long_spread(n, bp.resident_long));
+  cudaError_t e = cudaSuccess;
+  if (queues) e = cudaMemsetAsync(bp.d_counters, 0, kBatchCounters * sizeof(unsigned int), st);
   BatchParams p{};
   p.in = (const c32*)in;
   p.out = (c32*)out;
@@ -1185,8 +1215,6 @@ static b2f_status run_batch(const BatchPlan& bp, cudaStream_t st, const void* in
   p.line_off = bp.d_off;
   p.inverse = bp.direction == B2F_INVERSE ? 1u : 0u;
   p.tw = bp.d_tw;
-  const bool run_cl = (bp.n_cl || bp.n_big) && (parts & 2);
-  const bool run_cta = bp.n_cta && (parts & 1);
   cudaStream_t cl_stream = sequential ? st : bp.side;
   if (e == cudaSuccess && run_cl) {
     // long lines on a forked stream, concurrently with the CTA queue
@@ -1223,7 +1251,7 @@ static b2f_status run_batch(const BatchPlan& bp, cudaStream_t st, const void* in
   }
   // without cluster lines, the CTA queue runs on the forked stream,
   // concurrently with the long-line phases (no line is in both)
-  const bool cta_side = run_cta && !run_cl && !sequential && (parts & 4) && bp.lines_long;
+  const bool cta_side = run_cta && !run_cl && !sequential && run_long;
   if (e == cudaSuccess && cta_side) {
     e = cudaEventRecord(bp.fork, st);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(bp.side, bp.fork, 0);
@@ -1236,9 +1264,7 @@ static b2f_status run_batch(const BatchPlan& bp, cudaStream_t st, const void* in
     k_batch_cta<<<bp.grid_cta, kCtaThreads, bp.smem_cta, cta_side ? bp.side : st>>>(pt, bp.buf_cta);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess && (parts & 4) && bp.lines_long) {
-    launch_long(bp, st, in, out, -1, &e);
-  }
+  if (e == cudaSuccess && run_long) launch_long(bp, st, in, out, -1, &e);
   if (e == cudaSuccess && ((run_cl && !sequential) || cta_side)) {
     e = cudaEventRecord(bp.join, bp.side);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, bp.join, 0);
@@ -1567,6 +1593,11 @@ b2f_status line_batch_run(LineRegistry* reg, cudaStream_t st, const uint64_t* le
   std::vector<LongTask> lt[3];
   uint64_t scratch = 0;
   uint32_t buf_cta = 1, long_cap = 0, long_tab = 0;
+  std::vector<std::pair<uint32_t, uint64_t>> cta_lens;
+  for (auto& kv : by_idx)
+    if (reg->infos[kv.first]->d.kind <= BK_BLUE)
+      cta_lens.push_back({reg->infos[kv.first]->d.G, kv.second.size()});
+  const uint32_t cta_div = cta_divisor(cta_lens, reg->nsm);
   for (auto& kv : by_idx) {
     const LenInfo& li = *reg->infos[kv.first];
     const BatchLen& d = li.d;
@@ -1596,11 +1627,12 @@ b2f_status line_batch_run(LineRegistry* reg, cudaStream_t st, const uint64_t* le
       off_in.push_back(in_off[line]);
       off_out.push_back(out_off[line]);
     }
-    for (size_t s = 0; s < kv.second.size(); s += d.G) {
+    const uint32_t G = std::max(1u, d.G / cta_div);
+    for (size_t s = 0; s < kv.second.size(); s += G) {
       BatchTask t;
       t.len = (uint32_t)kv.first;
       t.first = first + (uint32_t)s;
-      t.count = (uint32_t)std::min<size_t>(d.G, kv.second.size() - s);
+      t.count = (uint32_t)std::min<size_t>(G, kv.second.size() - s);
       t.pad = 0;
       cta.push_back(t);
       cta_cost.push_back(li.cost * t.count);
