@@ -112,3 +112,10 @@ def test_tasks_of_short_lines(n, count, inverse):
     assert np.all(np.linalg.norm(y - ref, axis=1) <= 2e-6 * np.linalg.norm(ref, axis=1))
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert b.diagnostics()["cta_tasks"] >= min(count, 2 * sms, count * n // 1500)
+
+
+@pytest.mark.parametrize("n", [2, 16, 17, 18, 19, 47, 2731, 2777, 5600])
+def test_tasks_keep_their_share_of_shared_memory(n):
+    """A full task of any length fits a quarter of an SM (44 KiB of lines)."""
+    b = w.FftBatch(np.full(40000, n), np.arange(40000) * n)
+    assert 0 < b.diagnostics()["cta_smem"] <= 44 * 1024

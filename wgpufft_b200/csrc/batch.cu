@@ -433,11 +433,12 @@ static bool classify(uint64_t N, int32_t direction, int32_t normalization, size_
     sc = 1.0f / sqrtf((float)N);
   d.scale = sc;
   d.dN = make_fastdiv((uint32_t)N);
-  // bytes of a line in a CTA task (in place; up to 16 points two ping-pong
-  // buffers), with `extra` values beside the transform's buffer, and of a
-  // cluster rank's two buffers
-  const auto cta_bytes = [](uint64_t n, uint64_t extra = 0) {
-    return n <= 16 ? 2 * (size_t)ld_f32(n) * 8 : (size_t)(n + 17 + extra) * 8;
+  // bytes of a line in a CTA task: of a transform of n points in place, with
+  // `extra` values beside its buffer; of a mixed line of n points (up to 16
+  // two ping-pong buffers); and of a cluster rank's two buffers
+  const auto ip_bytes = [](uint64_t n, uint64_t extra = 0) { return (size_t)(n + 17 + extra) * 8; };
+  const auto cta_bytes = [&](uint64_t n) {
+    return n <= 16 ? 2 * (size_t)ld_f32(n) * 8 : ip_bytes(n);
   };
   const auto cl_bytes = [](uint64_t lbuf) { return 2 * (size_t)ld_f32(lbuf) * 8; };
   uint64_t n1 = 0;
@@ -470,7 +471,7 @@ static bool classify(uint64_t N, int32_t direction, int32_t normalization, size_
     }
   } else if (smooth) {
     set_long(li, N, N, n1, false);
-  } else if (is_prime_u64(N) && N >= 17 && is_smooth13(N - 1) && cta_bytes(N - 1, N + 2) <= cta_cap) {
+  } else if (is_prime_u64(N) && N >= 17 && is_smooth13(N - 1) && ip_bytes(N - 1, N + 2) <= cta_cap) {
     d.kind = BK_RADER;
     d.M = (uint32_t)(N - 1);
     const uint64_t g = primitive_root(N), ginv = mod_pow64(g, N - 2, N);
@@ -561,7 +562,7 @@ static bool classify(uint64_t N, int32_t direction, int32_t normalization, size_
     d.G = 1;
   } else if (d.kind == BK_MIXED || d.kind == BK_RADER || d.kind == BK_BLUE) {
     // lines that fill the CTA's share
-    const size_t line = d.kind == BK_RADER ? cta_bytes(N - 1, N + 2) : cta_bytes(d.M);
+    const size_t line = d.kind == BK_RADER ? ip_bytes(N - 1, N + 2) : cta_bytes(d.M);
     const uint64_t G = std::max<uint64_t>(1, std::min<uint64_t>(cta_cap / line, kBatchMaxG));
     d.G = (uint32_t)G;
   } else {
