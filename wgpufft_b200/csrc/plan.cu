@@ -475,9 +475,13 @@ struct Builder {
   bool fits_ip(uint64_t n, uint64_t extra = 0) const {
     return ip_on() && n > 16 && ip_bytes(n, extra) <= smem_budget;
   }
-  // Whether a mixed-radix line runs in one pass.
-  bool fits_lines(uint64_t n) const {
-    return fits_one_cta(n) || ((n & (n - 1)) != 0 && fits_ip(n));
+  // Whether a mixed-radix line of stride s runs in one pass.  A column that
+  // fills a CTA reads and writes 8 bytes (f64: 16) of every 32-byte sector, so
+  // that strided lines past the two-buffer limit take two passes, whatever
+  // their number: 2 x 20,000 points 43 -> 16 us, 2 x 28,000, 149 times, 194 ->
+  // 178 (rows are faster in one at any number: 28,800 points alone 56 -> 31).
+  bool fits_lines(uint64_t n, uint64_t s) const {
+    return fits_one_cta(n) || (s == 1 && (n & (n - 1)) != 0 && fits_ip(n));
   }
   // A Rader line of p points, a Bluestein convolution of m, in one pass.
   bool fits_rader(uint64_t p) const { return fits_ip(p - 1, p + 2) || fits_one_cta(p); }
@@ -649,8 +653,14 @@ static bool ip_shape(const Builder& b, Pass& ps, uint64_t inner_n, uint64_t grou
     G = seg;
     while (G > seg / 4 && G * line > most) G >>= 1;
     if (G == seg) G = std::max<uint64_t>(seg, third / line / seg * seg);
-    // a grid of fewer CTAs than SMs: narrower tiles
-    while (G > seg / 4 && G > 1 && (inner_n + G - 1) / G * groups < kSms) G >>= 1;
+    // a grid of fewer CTAs than SMs: narrower tiles, down to a sector's width
+    auto ctas_of = [&](uint64_t g) { return (inner_n + g - 1) / g * groups; };
+    while (G > seg / 4 && G > 1 && ctas_of(G) < kSms) G >>= 1;
+    // and, where a line alone is a CTA's work, to as few lines as give each SM
+    // at most one CTA: 16 columns of 4,099 points 47 -> 21 us, 4 of 9,240 26 ->
+    // 15 (past one CTA an SM 348 lines of 3,011 points go 35 -> 44)
+    if (line > third / 3)
+      while (G > 1 && ctas_of(G / 2) <= kSms) G >>= 1;
   } else {
     G = std::max<uint64_t>(1, third / line);
     G = std::min<uint64_t>(G, std::max<uint64_t>(1, inner_n * groups / (3 * kSms)));
@@ -675,22 +685,37 @@ static bool ip_shape(const Builder& b, Pass& ps, uint64_t inner_n, uint64_t grou
   return true;
 }
 
-// Starts an in-place pass: its schedule and twiddle table.
-static bool ip_begin(Builder& b, Pass& ps, IpKind kind, bool col, uint64_t N, uint64_t n,
-                     const LineIO& io, uint32_t flags, double scale) {
+// Starts an in-place pass of N points, n of them in memory, `extra` values a
+// line beside the transform's buffer: layout, schedule, shape and twiddle
+// table.  Lines that are contiguous in memory are rows, adjacent lines columns;
+// a single column a CTA runs as a strided row, whose odd-pitched sub-lines
+// keep the last stages free of bank conflicts (a column's last stage reads R
+// values apart): 16 columns of 10,007 points 67 -> 40 us, 128 of 12,601
+// (Rader) 470 -> 277.  Rader columns save a staged copy on the way out, which
+// is worth more than the conflicts of a last radix that is not a multiple of
+// four (8,009: 235 us as columns, 244 as rows).
+static bool ip_begin(Builder& b, Pass& ps, IpKind kind, uint64_t N, uint64_t n, uint64_t extra,
+                     const LineIO& io, uint64_t outer_n, uint32_t flags, double scale) {
+  bool col = io.in_inner == 1 && io.out_inner == 1 && io.in_es != 1;
+  if (!col && io.in_es != 1) return false;
   ps.kind = Pass::IP;
   ps.ip_kind = kind;
-  ps.ip_col = col;
   IpParams& q = ps.ip;
-  std::memset(&q, 0, sizeof(q));
-  q.io = io;
-  q.flags = flags;
-  q.scale = scale;
-  q.n = (uint32_t)n;
-  q.dn = make_fastdiv(q.n);
   std::vector<cd> tw;
-  if (!ip_schedule(N, !col, true, b.plan.prec == PREC_F32 ? 2 : 1, q.sc, ps.radices, tw))
-    return false;
+  for (;; col = false, flags &= ~(uint32_t)(PF_CFIRST_LOAD | PF_CFIRST_STORE)) {
+    ps.ip_col = col;
+    std::memset(&q, 0, sizeof(q));
+    q.io = io;
+    q.flags = flags;
+    q.scale = scale;
+    q.n = (uint32_t)n;
+    q.dn = make_fastdiv(q.n);
+    tw.clear();
+    if (!ip_schedule(N, !col, true, b.plan.prec == PREC_F32 ? 2 : 1, q.sc, ps.radices, tw) ||
+        !ip_shape(b, ps, io.inner_n, outer_n * io.mid_n, extra))
+      return false;
+    if (!col || q.G > 1 || (kind == IP_RADER && q.sc.st[q.sc.nst - 1].R % 4 != 0)) break;
+  }
   b.set_table(b.next_pass(), Builder::F_IP_TW, b.add_table(b.pack_complex(tw)));
   return true;
 }
@@ -701,13 +726,6 @@ static void ip_grid(Pass& ps, uint64_t outer_n) {
   if (q.io.tw_div == 0) q.io.tw_div = 1;
   q.d_tw = make_fastdiv(q.io.tw_div);
   ps.grid = (unsigned)(outer_n * q.io.mid_n * q.io.tiles);
-}
-
-// Whether the lines of an IO pattern are rows (contiguous points) or
-// columns (adjacent lines on both sides) for the in-place kernels.
-static bool ip_layout(const LineIO& io, bool* col) {
-  *col = io.in_inner == 1 && io.out_inner == 1 && io.in_es != 1;
-  return *col || io.in_es == 1;
 }
 
 // A convolution's spectrum in the order its frequencies take in the CTA.
@@ -736,14 +754,12 @@ static b2f_status add_lines_pass(Builder& b, int axis, uint64_t N, const LineIO&
   lp.flags = flags;
   lp.scale = scale;
   const bool p2 = try_pow2_pass(b, ps, outer_n);
-  bool col = false;
-  if (!p2 && b.fits_ip(N) && ip_layout(io, &col)) {
-    if (!ip_begin(b, ps, IP_LINES, col, N, N, io, flags, scale) || !ip_shape(b, ps, io.inner_n, outer_n * io.mid_n, 0))
-      return fail(B2F_ERR_UNSUPPORTED_LENGTH, "UnsupportedLength { len: " + std::to_string(N) + " }");
+  if (!p2 && b.fits_ip(N) && ip_begin(b, ps, IP_LINES, N, N, 0, io, outer_n, flags, scale)) {
     ip_grid(ps, outer_n);
     b.plan.passes.push_back(ps);
     return B2F_OK;
   }
+  if (!p2) ps.kind = Pass::LINES;
   std::vector<cd> tw;
   if (!b.make_schedule(N, lp.sch, ps.radices, tw))
     return fail(B2F_ERR_UNSUPPORTED_LENGTH, "UnsupportedLength { len: " + std::to_string(N) + " }");
@@ -807,11 +823,9 @@ static b2f_status add_rader_pass(Builder& b, int axis, uint64_t p, const LineIO&
   std::vector<unsigned char> bin(pin.size() * 4), bout(pout.size() * 4);
   std::memcpy(bin.data(), pin.data(), bin.size());
   std::memcpy(bout.data(), pout.data(), bout.size());
-  bool col = false;
   // p - 1 >= 16: the in-place kernels take every Rader length
-  if (b.ip_on() && p > 16 && b.fits_rader(p) && ip_layout(io, &col) &&
-      ip_begin(b, ps, IP_RADER, col, p - 1, p, io, flags, scale) &&
-      ip_shape(b, ps, io.inner_n, outer_n * io.mid_n, p + 2)) {
+  if (b.ip_on() && p > 16 && b.fits_rader(p) &&
+      ip_begin(b, ps, IP_RADER, p - 1, p, p + 2, io, outer_n, flags, scale)) {
     ip_grid(ps, outer_n);
     b.set_table(b.next_pass(), Builder::F_IP_PERM, b.add_table(std::move(bin)));
     b.set_table(b.next_pass(), Builder::F_IP_BHAT,
@@ -902,9 +916,7 @@ static b2f_status add_bluestein_pass(Builder& b, int axis, uint64_t N, const Lin
   ps.dst = dst;
   ps.label = "bluestein-fused-workgroup-stage";
   ps.route = "bluestein";
-  bool col = false;
-  if (b.fits_ip(M) && ip_layout(io, &col) &&
-      ip_begin(b, ps, IP_BLUE, col, M, N, io, flags, scale) && ip_shape(b, ps, io.inner_n, outer_n * io.mid_n, 0)) {
+  if (b.fits_ip(M) && ip_begin(b, ps, IP_BLUE, M, N, 0, io, outer_n, flags, scale)) {
     ip_grid(ps, outer_n);
     b.set_table(b.next_pass(), Builder::F_IP_BHAT,
                 b.add_table(b.pack_complex(ip_spectrum(ps.ip.sc, chirp_spectrum(N, M)))));
@@ -1171,7 +1183,7 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
   // Split into two passes of about sqrt(N), each a tile of many adjacent
   // columns (rows of hundreds of bytes), once enough columns exist.
   const bool split_strided = s >= 16 && N >= 2048;
-  if (b.fits_lines(N) && !split_strided) {
+  if (b.fits_lines(N, s) && !split_strided) {
     b2f_status st = add_lines_pass(b, axis, N, io, outer_n, flags, scale, src, out_buf,
                                    p2 ? "fused-pow2-workgroup-stage" : "fused-smooth-workgroup-stage",
                                    "mixed");
@@ -1353,9 +1365,11 @@ static b2f_status add_real_pass(Builder& b, bool r2c, uint64_t N0, uint64_t nlin
   // even N0 whose half is not a power of two (those have fixed-length kernels)
   if (even && (nfft & (nfft - 1)) != 0 && b.fits_ip(nfft, r2c ? nfft : 0)) {
     Pass pi = ps;
-    if (!ip_begin(b, pi, r2c ? IP_R2C : IP_C2R, false, nfft, nfft, LineIO{},
-                  (do_scale ? PF_SCALE : 0u) | (r2c ? 0u : PF_CONJ_OUT), scale) ||
-        !ip_shape(b, pi, nlines, 1, r2c ? nfft : 0))
+    LineIO io{};  // rows; the kernels know their layout
+    io.in_es = io.mid_n = 1;
+    io.inner_n = (uint32_t)nlines;
+    if (!ip_begin(b, pi, r2c ? IP_R2C : IP_C2R, nfft, nfft, r2c ? nfft : 0, io, 1,
+                  (do_scale ? PF_SCALE : 0u) | (r2c ? 0u : PF_CONJ_OUT), scale))
       return fail(B2F_ERR_UNSUPPORTED_LENGTH, "UnsupportedLength { len: " + std::to_string(N0) + " }");
     pi.ip.nlines = nlines;
     pi.ip.dn = make_fastdiv((uint32_t)(nfft / 2 + 1));  // R2C: pairs k <= N / 2
