@@ -1244,10 +1244,9 @@ static b2f_status add_complex_axis(Builder& b, int axis, AxisKind kind, uint64_t
     lp.tws_dn = (uint32_t)ta.size();
     b.set_table(idx, Builder::F_TWS_D, b.add_table(std::move(bytes)));
     if (lp.io.tw_div == 1) {
-      const RootProduct root(M);
-      std::vector<cd> t;
+      std::vector<cd> t;  // from the tables at hand: 2 sqrt(M) roots are 1.5 ms at M = 2^24
       for (uint64_t n = 0; n < lp.N; ++n)
-        for (uint64_t c = 0; c < lp.G; ++c) t.push_back(root(c * n % M));
+        for (uint64_t c = 0; c < lp.G; ++c) t.push_back(ta[c * n / L] * tb[c * n % L]);  // c n < M
       b.set_table(idx, Builder::F_TWS_T, b.add_table(b.pack_complex(t)));
     }
     ps.smem += (size_t)lp.N * b.cb();
