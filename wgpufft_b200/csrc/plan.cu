@@ -356,6 +356,8 @@ struct Builder {
   bool dry;           // planning only: no device allocations
   size_t smem_budget; // bytes of dynamic shared memory per CTA
   std::vector<std::pair<size_t, std::vector<unsigned char>>> pending;  // (alloc index, bytes)
+  // the device's; planning without one assumes a B200
+  uint64_t sms = 148, smem_sm = 228 * 1024;  // SMs, bytes of shared memory of each
 
   size_t cb() const { return complex_bytes(plan.prec); }
   int pad_shift() const { return plan.prec == PREC_F32 ? 4 : 3; }
@@ -625,7 +627,7 @@ static bool try_pow2_pass(Builder& b, Pass& ps, uint64_t outer_n) {
 // fit.
 static bool ip_shape(const Builder& b, Pass& ps, uint64_t inner_n, uint64_t groups,
                      uint64_t extra) {
-  constexpr uint64_t kSms = 148;
+  const uint64_t sms = b.sms;
   IpParams& q = ps.ip;
   const uint64_t N = q.sc.N;
   const size_t cb = b.cb();
@@ -655,15 +657,15 @@ static bool ip_shape(const Builder& b, Pass& ps, uint64_t inner_n, uint64_t grou
     if (G == seg) G = std::max<uint64_t>(seg, third / line / seg * seg);
     // a grid of fewer CTAs than SMs: narrower tiles, down to a sector's width
     auto ctas_of = [&](uint64_t g) { return (inner_n + g - 1) / g * groups; };
-    while (G > seg / 4 && G > 1 && ctas_of(G) < kSms) G >>= 1;
+    while (G > seg / 4 && G > 1 && ctas_of(G) < sms) G >>= 1;
     // and, where a line alone is a CTA's work, to as few lines as give each SM
     // at most one CTA: 16 columns of 4,099 points 47 -> 21 us, 4 of 9,240 26 ->
     // 15 (past one CTA an SM 348 lines of 3,011 points go 35 -> 44)
     if (line > third / 3)
-      while (G > 1 && ctas_of(G / 2) <= kSms) G >>= 1;
+      while (G > 1 && ctas_of(G / 2) <= sms) G >>= 1;
   } else {
     G = std::max<uint64_t>(1, third / line);
-    G = std::min<uint64_t>(G, std::max<uint64_t>(1, inner_n * groups / (3 * kSms)));
+    G = std::min<uint64_t>(G, std::max<uint64_t>(1, inner_n * groups / (3 * sms)));
   }
   while (G > 1 && G * line > b.smem_budget) --G;
   G = std::min<uint64_t>(G, std::max<uint64_t>(inner_n, 1));
@@ -675,8 +677,8 @@ static bool ip_shape(const Builder& b, Pass& ps, uint64_t inner_n, uint64_t grou
   // the CTAs that share an SM (by shared memory and by the grid) share its
   // threads; no more threads than the widest stage has butterflies
   const uint64_t grid = std::max<uint64_t>(1, (inner_n + G - 1) / G * groups);
-  uint64_t ctas = std::max<uint64_t>(1, (228 * 1024) / (ps.smem + 1024));
-  ctas = std::min<uint64_t>(std::min<uint64_t>(ctas, 16), (grid + kSms - 1) / kSms);
+  uint64_t ctas = std::max<uint64_t>(1, b.smem_sm / (ps.smem + 1024));
+  ctas = std::min<uint64_t>(std::min<uint64_t>(ctas, 16), (grid + sms - 1) / sms);
   uint32_t rmin = q.sc.R0 > 1 ? q.sc.R0 : 16;
   for (uint32_t s = 0; s < q.sc.nst; ++s) rmin = std::min(rmin, q.sc.st[s].R);
   uint64_t T = ip_threads_per_sm(b.plan.prec) / ctas / 32 * 32;
@@ -1687,6 +1689,10 @@ b2f_status create_plan(const Config& cfg_in, int32_t kind, int device, Plan** ou
     if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
       v = 48 * 1024;
     b.smem_budget = (size_t)v;
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && v > 0)
+      b.sms = (uint64_t)v;
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) == cudaSuccess && v > 0)
+      b.smem_sm = (uint64_t)v;
   }
   const size_t cbytes = complex_bytes(plan->prec);
   const size_t sbytes = plan->prec == PREC_F64 ? 8 : 4;
@@ -1726,9 +1732,7 @@ b2f_status create_plan(const Config& cfg_in, int32_t kind, int device, Plan** ou
       ps.tc_inverse = inverse;
       ps.threads = 256;
       ps.smem = 192 * 1024;
-      int nsm = 148;
-      if (!dry) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-      ps.grid = (unsigned)std::min<uint64_t>((uint64_t)nsm, (ps.tc_nlines + 31) / 32);
+      ps.grid = (unsigned)std::min<uint64_t>(b.sms, (ps.tc_nlines + 31) / 32);
       const std::vector<float> tab = dft64_tc_table();
       std::vector<unsigned char> tb(tab.size() * 4);
       std::memcpy(tb.data(), tab.data(), tb.size());
