@@ -611,23 +611,36 @@ static uint32_t cta_divisor(const std::vector<std::pair<uint32_t, uint64_t>>& le
 
 // CTAs of a long phase: tasks that are dealt out have one each as far as they
 // fit, tasks of the queue one a chunk.
-static bool long_spread(uint64_t tasks, unsigned resident) {
+static bool long_dealt(uint64_t tasks, unsigned resident) {
   return tasks <= (uint64_t)kLongSpread * resident;
 }
 static unsigned long_grid(uint64_t tasks, unsigned resident) {
   return (unsigned)std::min<uint64_t>(
-      resident, long_spread(tasks, resident) ? tasks : (tasks + kLongChunk - 1) / kLongChunk);
+      resident, long_dealt(tasks, resident) ? tasks : (tasks + kLongChunk - 1) / kLongChunk);
+}
+
+// The kernels of the phases, tasks from the queue and dealt out.
+using LongKernel = void (*)(LongParams);
+static const LongKernel kLongKernels[2][3] = {
+    {k_long_pass<1, false>, k_long_pass<2, false>, k_long_pass<3, false>},
+    {k_long_pass<1, true>, k_long_pass<2, true>, k_long_pass<3, true>}};
+
+// Opts them in to `smem` bytes; *per_sm: CTAs that fit an SM.
+static cudaError_t set_long_smem(size_t smem, int* per_sm) {
+  for (const auto& phases : kLongKernels)
+    for (LongKernel k : phases) {
+      const cudaError_t e = set_smem(k, smem);
+      if (e != cudaSuccess) return e;
+    }
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kLongKernels[0][1], kLongThreads, smem);
 }
 
 // Launches phase ph (0..2) over lp.ntasks tasks.
 static cudaError_t launch_long_phase(LongParams& lp, uint32_t ph, unsigned resident, size_t smem,
                                      cudaStream_t st) {
   lp.phase = ph + 1;
-  lp.spread = long_spread(lp.ntasks, resident);
-  const unsigned grid = long_grid(lp.ntasks, resident);
-  if (ph == 0) k_long_pass<1><<<grid, kLongThreads, smem, st>>>(lp);
-  else if (ph == 1) k_long_pass<2><<<grid, kLongThreads, smem, st>>>(lp);
-  else k_long_pass<3><<<grid, kLongThreads, smem, st>>>(lp);
+  kLongKernels[long_dealt(lp.ntasks, resident)][ph]<<<long_grid(lp.ntasks, resident), kLongThreads,
+                                                      smem, st>>>(lp);
   return cudaGetLastError();
 }
 
@@ -1092,12 +1105,9 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
   }
   if (n_long_lines) {
     bp->smem_long = ((size_t)bp->long_cap + bp->long_tab) * 8;
-    if (set_smem(k_long_pass<1>, bp->smem_long) != cudaSuccess ||
-        set_smem(k_long_pass<2>, bp->smem_long) != cudaSuccess ||
-        set_smem(k_long_pass<3>, bp->smem_long) != cudaSuccess)
-      return fail(B2F_ERR_DEVICE, "long-line kernel shared memory");
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_long_pass<2>, kLongThreads, bp->smem_long);
+    if (set_long_smem(bp->smem_long, &per_sm) != cudaSuccess)
+      return fail(B2F_ERR_DEVICE, "long-line kernel shared memory");
     per_sm = std::max(per_sm, 1);
     bp->resident_long = (unsigned)nsm * per_sm;
     for (uint32_t n : bp->long_count) bp->grid_long = std::max(bp->grid_long, long_grid(n, bp->resident_long));
@@ -1206,7 +1216,7 @@ static b2f_status run_batch(const BatchPlan& bp, cudaStream_t st, const void* in
   // launches with a CTA for every task, or whose tasks are dealt out, leave
   // the counters alone
   bool queues = run_cl || (run_cta && bp.grid_cta < bp.n_cta);
-  for (uint32_t n : bp.long_count) queues = queues || (run_long && !long_spread(n, bp.resident_long));
+  for (uint32_t n : bp.long_count) queues = queues || (run_long && !long_dealt(n, bp.resident_long));
   cudaError_t e = cudaSuccess;
   if (queues) e = cudaMemsetAsync(bp.d_counters, 0, kBatchCounters * sizeof(unsigned int), st);
   BatchParams p{};
@@ -1696,12 +1706,8 @@ b2f_status line_batch_run(LineRegistry* reg, cudaStream_t st, const uint64_t* le
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&reg->cta_per_sm, k_batch_cta, kCtaThreads, smem_cta);
   }
   if (e == cudaSuccess && nlt && smem_long > reg->long_smem_set) {
-    e = set_smem(k_long_pass<1>, smem_long);
-    if (e == cudaSuccess) e = set_smem(k_long_pass<2>, smem_long);
-    if (e == cudaSuccess) e = set_smem(k_long_pass<3>, smem_long);
+    e = set_long_smem(smem_long, &reg->long_per_sm);
     reg->long_smem_set = smem_long;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&reg->long_per_sm, k_long_pass<2>, kLongThreads,
-                                                  smem_long);
   }
   if (e == cudaSuccess && !cta.empty()) {
     BatchParams pt{};

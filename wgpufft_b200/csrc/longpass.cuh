@@ -109,7 +109,6 @@ struct LongParams {
   uint32_t phase;    // 1: column pass, 2: row pass, 3: Bluestein inverse columns
   uint32_t inverse;
   uint32_t cap;      // complex elements of the data buffer
-  uint32_t spread;   // tasks are dealt out, not taken from the queue
   unsigned int* counter;  // work queue: chunks of kLongChunk tasks handed out in order
 };
 
@@ -345,7 +344,8 @@ FFT_D void long_task(const LongParams& p, const LongLenDesc& d, const LongTask& 
 }
 
 // Persistent kernel of one long-line phase PH (= p.phase).  Tasks that are
-// not dealt out (p.spread) come in chunks of kLongChunk consecutive ones from
+// not DEALT out (kernels of their own: asking at run time costs the 20,000
+// mixed lines 1 %) come in chunks of kLongChunk consecutive ones from
 // a work queue (one atomicAdd per chunk), claimed a chunk ahead: the claim for
 // the CTA's chunk c + 1 is issued when it starts using chunk c and its result
 // is stored after that iteration's task, so the atomic's latency is hidden
@@ -353,7 +353,7 @@ FFT_D void long_task(const LongParams& p, const LongLenDesc& d, const LongTask& 
 // descriptor of task k + 2 (a ring of three) and the record of task k + 3 (a
 // ring of four).
 // Dynamic shared memory: p.cap values of data, then the tables.
-template <uint32_t PH>
+template <uint32_t PH, bool DEALT>
 __global__ void __launch_bounds__(kLongThreads, 4) k_long_pass(const __grid_constant__ LongParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ LongLenDesc s_len[3];
@@ -367,11 +367,11 @@ __global__ void __launch_bounds__(kLongThreads, 4) k_long_pass(const __grid_cons
   // the CTA's k-th task (of the queue: its chunk claimed and visible); kNone
   // from the first one past the end (the queue hands out chunks in increasing order)
   auto task_of = [&](uint32_t k) -> uint32_t {
-    const uint64_t t = p.spread ? blockIdx.x + (uint64_t)k * gridDim.x
-                                : (uint64_t)s_chunk[(k / kLongChunk) & 3] + k % kLongChunk;
+    const uint64_t t = DEALT ? blockIdx.x + (uint64_t)k * gridDim.x
+                             : (uint64_t)s_chunk[(k / kLongChunk) & 3] + k % kLongChunk;
     return t < p.ntasks ? (uint32_t)t : kNone;
   };
-  if (tid == 0 && !p.spread) {
+  if (tid == 0 && !DEALT) {
     s_chunk[0] = atomicAdd(p.counter, 1u) * kLongChunk;
     s_chunk[1] = atomicAdd(p.counter, 1u) * kLongChunk;
   }
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(kLongThreads, 4) k_long_pass(const __grid_cons
     __syncthreads();  // task k's and k + 1's descriptors and k + 2's record have landed, and
                       // every thread is past task k - 1
     // task k + 3 opens chunk c = (k + 3) / kLongChunk: claim chunk c + 1
-    const bool claim = tid == 0 && !p.spread && (k + 3) % kLongChunk == 0;
+    const bool claim = tid == 0 && !DEALT && (k + 3) % kLongChunk == 0;
     const uint32_t claimed = claim ? atomicAdd(p.counter, 1u) * kLongChunk : 0u;
     const LongLenDesc& d = s_len[k % 3];
     const LongTask& ln = s_task[k & 3];
