@@ -592,21 +592,25 @@ static cudaError_t set_smem(K kernel, size_t smem) {
                               std::max<int>(room, (int)smem));
 }
 
-// What the lines of a CTA task (G of each length, filling the CTA's share of
-// the shared memory) are divided by, 1, 2 or 4, until the batch has two tasks
-// an SM: a task's loads, stages and stores follow one another, so that few
-// full tasks leave the chip idle (148 lines of 2,600 points as 74 tasks 16.4
-// us, as 148 12.3; 300 of 32 points as 3 tasks 12.3, as 11 8.2).  Dividing by
-// 8, or until there are four an SM, costs batches of many short lines more
-// than it gives (20,000 of 32 points 12.4 -> 16.2 us, 600 of 1,009 21 -> 27).
-static uint32_t cta_divisor(const std::vector<std::pair<uint32_t, uint64_t>>& lens, int nsm) {
-  uint32_t div = 1;
-  for (; div < 4; div *= 2) {
+// Lines of a CTA task: G of each length fill the CTA's share of the shared
+// memory; they are divided by up to four (`halves` / 2, in steps of a half at
+// first) until the batch has two tasks an SM.  A task's loads, stages and stores
+// follow one another, so that few full tasks leave the chip idle (148 lines of
+// 2,600 points as 74 tasks 16.4 us, as 148 12.3; 300 of 32 points as 3 tasks
+// 12.3, as 11 8.2).  Dividing by eight, or until there are four an SM, costs
+// batches of many short lines more than it gives (20,000 of 32 points 12.4 ->
+// 16.2 us, 600 of 1,009 21 -> 27).
+static uint32_t cta_lines(uint32_t G, uint32_t halves) { return std::max(1u, 2 * G / halves); }
+static uint32_t cta_halves(const std::vector<std::pair<uint32_t, uint64_t>>& lens, int nsm) {
+  for (uint32_t halves : {2u, 3u, 4u, 6u}) {
     uint64_t tasks = 0;
-    for (const auto& [G, lines] : lens) tasks += (lines + std::max(1u, G / div) - 1) / std::max(1u, G / div);
-    if (tasks >= 2ull * nsm) break;
+    for (const auto& [G, lines] : lens) {
+      const uint32_t g = cta_lines(G, halves);
+      tasks += (lines + g - 1) / g;
+    }
+    if (tasks >= 2ull * nsm) return halves;
   }
-  return div;
+  return 8;
 }
 
 // CTAs of a long phase: tasks that are dealt out have one each as far as they
@@ -880,7 +884,7 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
   std::vector<std::pair<uint32_t, uint64_t>> cta_lens;
   for (size_t li = 0; li < lens_list.size(); ++li)
     if (infos[li].d.kind <= BK_BLUE) cta_lens.push_back({infos[li].d.G, by_len[lens_list[li]].size()});
-  const uint32_t cta_div = cta_divisor(cta_lens, nsm);
+  const uint32_t halves = cta_halves(cta_lens, nsm);
   std::vector<uint64_t> sorted_off;
   std::vector<BatchTask> cta_tasks, cl_tasks, big_tasks, cta_ch_tasks;
   std::vector<double> cta_cost, cl_cost, big_cost, cta_ch_cost;
@@ -953,7 +957,7 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
       }
       continue;
     }
-    const uint32_t G = std::max(1u, d.G / cta_div);
+    const uint32_t G = cta_lines(d.G, halves);
     for (size_t s = 0; s < ls.size(); s += G) {
       const BatchTask t = make(s, std::min<size_t>(ls.size(), s + G), 0);
       cta_tasks.push_back(t);
@@ -1608,7 +1612,7 @@ b2f_status line_batch_run(LineRegistry* reg, cudaStream_t st, const uint64_t* le
   for (auto& kv : by_idx)
     if (reg->infos[kv.first]->d.kind <= BK_BLUE)
       cta_lens.push_back({reg->infos[kv.first]->d.G, kv.second.size()});
-  const uint32_t cta_div = cta_divisor(cta_lens, reg->nsm);
+  const uint32_t halves = cta_halves(cta_lens, reg->nsm);
   for (auto& kv : by_idx) {
     const LenInfo& li = *reg->infos[kv.first];
     const BatchLen& d = li.d;
@@ -1638,7 +1642,7 @@ b2f_status line_batch_run(LineRegistry* reg, cudaStream_t st, const uint64_t* le
       off_in.push_back(in_off[line]);
       off_out.push_back(out_off[line]);
     }
-    const uint32_t G = std::max(1u, d.G / cta_div);
+    const uint32_t G = cta_lines(d.G, halves);
     for (size_t s = 0; s < kv.second.size(); s += G) {
       BatchTask t;
       t.len = (uint32_t)kv.first;

@@ -205,39 +205,18 @@ struct BatchChirpStore {
   }
 };
 
-// v = f(e), then g(e, v), over e < total, the loads of eight values a thread
-// in flight together.
-template <class F, class Gf>
-FFT_D void batch_copy(uint32_t total, uint32_t tid, uint32_t T, F f, Gf g) {
-  constexpr int U = 8;
-#pragma unroll 1
-  for (uint32_t e = tid; e < total; e += U * T) {
-    c32 v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) v[u] = e + u * T < total ? f(e + u * T) : czero<float>();
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (e + u * T < total) g(e + u * T, v[u]);
-  }
-}
-
 // Lines of up to 16 points: one or two ping-pong stages.
 FFT_D void batch_tiny(const BatchParams& bp, const BatchLen& L, const int64_t* base,
                       const int64_t* obase, uint32_t cnt, c32* A, c32* B, uint32_t tid, uint32_t T) {
   constexpr int PAD = PadOf<float>::value;
   const uint32_t N = L.N, LD = L.LD;
   const bool inv = bp.inverse;
-  batch_copy(
-      cnt * N, tid, T,
-      [&](uint32_t e) {
-        const uint32_t c = fdiv(e, L.dN);
-        return bp.in[base[c] + (e - c * N)];
-      },
-      [&](uint32_t e, c32 v) {
-        const uint32_t c = fdiv(e, L.dN);
-        if (inv) v.im = -v.im;
-        A[c * LD + pidx<PAD>(e - c * N)] = v;
-      });
+  for (uint32_t e = tid; e < cnt * N; e += T) {
+    const uint32_t c = fdiv(e, L.dN), n = e - c * N;
+    c32 v = bp.in[base[c] + n];
+    if (inv) v.im = -v.im;
+    A[c * LD + pidx<PAD>(n)] = v;
+  }
   __syncthreads();
   const c32* r = fft_lines_smem<float>(A, B, L.sch, cnt, LD, tid, T, bp.tw);
   const float sc = L.scale;
@@ -272,18 +251,13 @@ FFT_D void batch_lines(const BatchParams& bp, const BatchLen& L, const int64_t* 
     c32* stage = buf + cnt * L.ip.LDl;
     c32* x0 = stage + cnt * n;
     c32* X0 = x0 + cnt;
-    batch_copy(
-        cnt * n, tid, T,
-        [&](uint32_t e) {
-          const uint32_t c = fdiv(e, L.dN);
-          return bp.in[base[c] + (e - c * n)];
-        },
-        [&](uint32_t e, c32 v) {
-          const uint32_t c = fdiv(e, L.dN);
-          if (inv) v.im = -v.im;
-          stage[e] = v;
-          if (e == c * n) x0[c] = v;
-        });
+    for (uint32_t e = tid; e < cnt * n; e += T) {
+      const uint32_t c = fdiv(e, L.dN), i = e - c * n;
+      c32 v = bp.in[base[c] + i];
+      if (inv) v.im = -v.im;
+      stage[e] = v;
+      if (i == 0) x0[c] = v;
+    }
     __syncthreads();
     ip.first(IpGather<float, false>{stage, L.perm, n, 0});
     ip.forward_mids();
@@ -332,10 +306,14 @@ __global__ void __launch_bounds__(256, 4) k_batch_cta(const __grid_constant__ Ba
   uint32_t s_len_idx = 0xFFFFFFFFu;  // length descriptor currently in s_len (same in every thread)
   c32* A = reinterpret_cast<c32*>(smem_raw);
   const uint32_t tid = threadIdx.x, T = blockDim.x;
-  // the first task is the CTA's own (no atomic to wait for, and no counter to
-  // zero where there are no more tasks than CTAs), the rest come from the queue
+  // a task for every CTA: no atomic to wait for, no counter to zero
   const bool queue = gridDim.x < bp.ntasks;
   uint32_t t = blockIdx.x;
+  if (queue) {
+    if (tid == 0) s_task = atomicAdd(bp.counter, 1u);
+    __syncthreads();
+    t = s_task;
+  }
   while (t < bp.ntasks) {
     const BatchTask task = bp.tasks[t];
     if (task.len != s_len_idx) copy_words(&s_len, bp.lens + task.len, tid, T);
@@ -362,7 +340,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_cta(const __grid_constant__ Ba
     if (!queue) break;
     if (tid == 0) s_task = next;
     __syncthreads();
-    t = gridDim.x + s_task;
+    t = s_task;
   }
 }
 
