@@ -596,8 +596,8 @@ static cudaError_t set_smem(K kernel, size_t smem) {
 // memory; they are divided by up to four (`halves` / 2, in steps of a half at
 // first) until the batch has two tasks an SM.  A task's loads, stages and stores
 // follow one another, so that few full tasks leave the chip idle (148 lines of
-// 2,600 points as 74 tasks 16.4 us, as 148 12.3; 300 of 32 points as 3 tasks
-// 12.3, as 11 8.2).  Dividing by eight, or until there are four an SM, costs
+// 2,600 points as 74 tasks 16.4 us, as 148 12.3, and 8.9 without a counter to
+// zero; 300 of 32 points as 3 tasks 12.3, as 11 8.2, and 4.7).  Dividing by eight, or until there are four an SM, costs
 // batches of many short lines more than it gives (20,000 of 32 points 12.4 ->
 // 16.2 us, 600 of 1,009 21 -> 27).
 static uint32_t cta_lines(uint32_t G, uint32_t halves) { return std::max(1u, 2 * G / halves); }
@@ -718,7 +718,8 @@ static b2f_status create_batch(const uint64_t* lengths, const uint64_t* offsets,
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   // A batch with few long lines takes smaller tasks, down to about 1,000
   // values (four a thread), until a phase has two tasks an SM, half of what
-  // is resident: 64 lines of 10,007 points 41 -> 33 us, 16 of 65,521 56 -> 48.
+  // is resident: 64 lines of 10,007 points 41 -> 33 us, 16 of 65,521 56 -> 48
+  // (27 and 42 now).
   // Halving them until every resident CTA has two instead leaves batches of a
   // few hundred lines with twice the stage rounds (64 x 10,007 55 us, 370
   // lines of up to 15,000 points 54 against 40).  (The values a task holds do

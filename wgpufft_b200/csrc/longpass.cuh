@@ -31,11 +31,11 @@
 // the next task's data or tables into L2 ahead cost its instructions and 3 %
 // instead).
 //
-// What bounds it: instruction issue, 335 thread instructions per point of
-// the 20,000-line mixed workload (540 with the earlier ping-pong stages and
-// 16 warps an SM) at 44-50 % of the issue slots, behind loads, barriers and,
-// as neighbouring tasks run other radices, instruction fetch.  That workload:
-// 4.32 -> 3.14 ms; 512 x 65536: 404 -> 244 us; 512 x 65521 (Bluestein): 1994
+// What bounds it: instruction issue, 339 thread instructions per point of
+// the first 4,000 lines of the mixed workload (540 with the earlier ping-pong
+// stages and 16 warps an SM) at 43-46 % of the issue slots, behind loads,
+// barriers and, as neighbouring tasks run other radices, instruction fetch.
+// All 20,000 lines: 4.32 -> 3.08 ms; 512 x 65536: 404 -> 244 us; 512 x 65521 (Bluestein): 1994
 // -> 1026; 1118 x 30011: 1676 -> 853; 6706 x 5003: 2122 -> 931.
 #pragma once
 #include "batch.cuh"
@@ -48,8 +48,8 @@ constexpr uint32_t kLongChunk = 4;  // consecutive tasks per work-queue claim
 // Tasks a resident CTA up to which they are dealt out.  A CTA holds four to
 // eight tasks of the queue from its start, so that small batches ran theirs
 // one after the other in a quarter of the CTAs: us from the queue / dealt out,
-// one line of 3,001 points 55.6 / 22.7, 300 of 6,000 67.7 / 28.7, 64 of 65,536
-// 87.3 / 45.9.  With 20 to 32 tasks a CTA dealing is still ahead (20,000 lines
+// without a counter to zero, one line of 3,001 points 56.9 / 19.0, 300 of 6,000
+// 67.8 / 22.8, 64 of 65,536 87.7 / 39.6.  With 20 to 32 tasks a CTA dealing is still ahead (20,000 lines
 // of up to 15,000 points 783 / 752, 2,400 of 20,000 442 / 412); at 40 to 65
 // the queue is (10,000 of up to 65,536 1597 / 1631, 4,800 of 10,007 1273 /
 // 1316), at 100 neither (20,000 of up to 65,536).

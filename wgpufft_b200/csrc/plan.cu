@@ -648,7 +648,8 @@ static bool ip_shape(const Builder& b, Pass& ps, uint64_t inner_n, uint64_t grou
   if (across) {
     // Whole 128-byte segments where they fit at all: 1080-point columns take
     // 54 us as one CTA of 16 lines and 1024 threads an SM, 58 as three of 8,
-    // 70 as six of 4.  A convolution's phases overlap across three CTAs
+    // 70 as six of 4; 480, 1200 and 1750 points 54, 47 and 54 against 66, 56 and
+    // 60 with 8 lines, though 600, 900 and 1500 are 5 to 13 % better with 8.  A convolution's phases overlap across three CTAs
     // instead (1009: 96 us with 4 lines in 63 KB, 105 with 8 in 126 KB), if
     // that leaves a 32-byte sector.
     const size_t most = ps.ip_kind == IP_LINES ? b.smem_budget : third;

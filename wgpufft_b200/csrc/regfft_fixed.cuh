@@ -119,7 +119,7 @@ FFT_D void fx_stages(cpx<S> (&v)[E], cpx<S>* line, uint32_t t, const cpx<S>* __r
 // otherwise a table shared by every tile, read with adjacent columns side by
 // side.  Looking W_M^{row n} up in the two sqrt(M) tables for every value
 // scatters each load over up to 32 cache lines: one line of 2^24 points
-// 212 -> 201 us, 4096 x 2048 100 -> 93 us, 256 x 65536 132 -> 126 us.
+// 212 -> 201 us, 4096 x 2048 92 -> 90 us, 256 x 65536 132 -> 126 us.
 // Tiles of 512-point columns (8 adjacent rows) are faster with the two
 // tables (64 x 2^18 161 against 167 us), so the planner builds T2 for up to
 // 256 points; kernels of their own (TT), as the code costs passes without a
